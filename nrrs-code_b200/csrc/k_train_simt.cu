@@ -27,8 +27,6 @@ namespace nrrs {
 namespace {
 
 constexpr int kTT = 128;           // threads per CTA of the training kernels
-constexpr int kChunk = 2048;       // samples per weight-gradient partial
-constexpr int kMaxJobs = 8;
 
 struct TrainArgs {
     VertexPtrs v;
@@ -506,79 +504,222 @@ cudaError_t launch_loss_sums(const LossWeights& w, uint32_t n, const float* erro
 namespace {
 
 // ---- weight gradients: dW[o][k] = sum_i D[o][i] * A[k][i] over the batch ----
+// One job is one output tile (at most 64 x 64) of one layer; a CTA computes it over one sample
+// chunk. Tile shapes are thread grids TY x TX of RU x 4 outputs each (kWShapes below); a thread
+// grid smaller than the CTA is repeated as sample groups, whose sums are added at the end in
+// group order.
 struct WJob {
-    uint32_t d_row, a_row;   // first scratch row of the deltas / activations
-    uint32_t M, N;           // outputs x inputs actually stored
-    uint32_t ldw;            // input width of the layer (row stride of W, >= N)
-    uint32_t out;            // offset of the layer in the MLP gradient vector
+    uint32_t d_row, a_row;   // first scratch row of the tile's deltas / activations
+    uint32_t M, N;           // rows that exist in the scratch (the rest of the tile is zero)
+    uint32_t store_n;        // columns written: N and the layer's zero input lanes
+    uint32_t ldw;            // input width of the layer (row stride of W)
+    uint32_t out;            // offset of the tile in the MLP gradient vector
+    uint32_t shape;          // index into kWShapes
 };
+constexpr int kMaxJobs = 32;
 
 struct WGradArgs {
     const float* act;
-    uint32_t ld, n, chunks;
+    uint32_t ld, n;
+    uint32_t chunk;          // samples per chunk, a multiple of kWS
     float* partial;          // [chunks][total]
     uint32_t total;          // MLP gradient length
-    int32_t njobs;
     WJob job[kMaxJobs];
 };
 
-// one CTA: one job x one 64x64 output tile x one sample chunk
-__global__ void __launch_bounds__(256) k_wgrad(const __grid_constant__ WGradArgs a) {
-    __shared__ float sD[32][65];
-    __shared__ float sA[32][65];
-    const WJob& j = a.job[blockIdx.z];
-    const uint32_t tiles_n = (j.N + 63) / 64;
-    const uint32_t tm = blockIdx.y / tiles_n, tn = blockIdx.y % tiles_n;
-    if (tm * 64 >= j.M || tn * 64 >= j.N) return;
-    const uint32_t m0 = tm * 64, n0 = tn * 64;
-    const uint32_t i0 = blockIdx.x * kChunk;
-    const uint32_t i1 = min(a.n, i0 + kChunk);
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    float acc[4][4] = {};
-    for (uint32_t ib = i0; ib < i1; ib += 32) {
-        // stage 32 samples of 64 delta rows and 64 activation rows (samples contiguous)
-        for (int e = threadIdx.x; e < 32 * 64; e += 256) {
-            const int r = e / 32, s = e % 32;
-            const uint32_t i = ib + s;
-            const bool ok_i = i < i1;
-            sD[s][r] = (ok_i && m0 + r < j.M) ? a.act[(size_t)(j.d_row + m0 + r) * a.ld + i] : 0.f;
-            sA[s][r] = (ok_i && n0 + r < j.N) ? a.act[(size_t)(j.a_row + n0 + r) * a.ld + i] : 0.f;
-        }
-        __syncthreads();
-#pragma unroll 8
-        for (int s = 0; s < 32; ++s) {
-            float d[4], x[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) d[u] = sD[s][ty * 4 + u];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) x[u] = sA[s][tx * 4 + u];
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int w = 0; w < 4; ++w) acc[u][w] = fmaf(d[u], x[w], acc[u][w]);
-        }
-        __syncthreads();
+constexpr int kWThr = 256;
+constexpr int kWS = 64;          // samples per stage
+constexpr int kWStages = 3;
+// row pitch of a stage: 64 samples and 4 floats, so that rows r, r+1, .. r+7 start 4 banks apart
+// and eight 16-byte reads of consecutive rows take one pass
+constexpr int kWPitch = kWS + 4;
+constexpr int kWRows = 128;      // largest tile: 64 delta + 64 activation rows
+constexpr size_t kWSmem = sizeof(float) * (size_t)kWStages * kWRows * kWPitch;
+
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b,
+                                                   unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
+// The whole (job, chunk): rows arrive as 16-byte cp.async copies (samples past the chunk's end
+// zero-filled), three stages deep; a thread reads 4 samples of its RU delta and 4 activation rows
+// as 16-byte words and adds the products of the even and odd samples as FP32 pairs (two FMAs per
+// issue slot).
+template <int RU, int TY, int TX>
+__device__ __forceinline__ void wgrad_tile(const WGradArgs& a, const WJob& j, float* sm,
+                                           uint32_t i0, uint32_t i1, float* out) {
+    constexpr int TM = RU * TY, TN = 4 * TX, ROWS = TM + TN;
+    constexpr int G = TY * TX, GROUPS = kWThr / G;
+    static_assert(ROWS <= kWRows && kWThr % G == 0 && GROUPS <= kWS / 4, "tile shape");
+    static_assert(GROUPS * TM * TN <= kWStages * kWRows * kWPitch, "group sums fit the stages");
+    const int tid = threadIdx.x;
+    const int tx = tid % TX, ty = (tid / TX) % TY, grp = tid / G;
+    constexpr int kStage = ROWS * kWPitch;
+    // rows of the tile that no layer row backs stay zero in every stage
+    for (int e = tid; e < kWStages * ROWS * (kWS / 4); e += kWThr) {
+        const int st = e / (ROWS * (kWS / 4)), r = (e / (kWS / 4)) % ROWS, q = e % (kWS / 4);
+        const bool live = r < TM ? (uint32_t)r < j.M : (uint32_t)(r - TM) < j.N;
+        if (!live)
+            *reinterpret_cast<float4*>(sm + st * kStage + r * kWPitch + 4 * q) =
+                make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    float* out = a.partial + (size_t)blockIdx.x * a.total + j.out;
+    const uint32_t stages = (i1 - i0 + kWS - 1) / kWS;
+    auto issue = [&](uint32_t s) {
+        if (s < stages) {
+            float* dst = sm + (s % kWStages) * kStage;
+            const uint32_t ib = i0 + s * kWS;
+            for (int e = tid; e < ROWS * (kWS / 4); e += kWThr) {
+                const int r = e / (kWS / 4), q = e % (kWS / 4);
+                const bool d = r < TM;
+                const uint32_t rr = d ? (uint32_t)r : (uint32_t)(r - TM);
+                if (rr >= (d ? j.M : j.N)) continue;
+                const uint32_t i = ib + 4 * q;
+                const uint32_t left = i < i1 ? i1 - i : 0u;
+                simt::cp_async16_n(dst + r * kWPitch + 4 * q,
+                                   a.act + (size_t)((d ? j.d_row : j.a_row) + rr) * a.ld +
+                                       (left ? i : i0),
+                                   left >= 4u ? 16u : 4u * left);
+            }
+        }
+        simt::cp_async_commit();
+    };
+    unsigned long long acc[RU][4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        const uint32_t m = m0 + ty * 4 + u;
-        if (m >= j.M) continue;
+    for (int u = 0; u < RU; ++u)
+#pragma unroll
+        for (int w = 0; w < 4; ++w) acc[u][w] = 0ull;
+#pragma unroll
+    for (int s = 0; s < kWStages - 1; ++s) issue(s);
+    for (uint32_t s = 0; s < stages; ++s) {
+        simt::cp_async_wait<kWStages - 2>();
+        __syncthreads();   // stage s has landed for everyone, and stage s - 1 is free
+        issue(s + kWStages - 1);
+        const float* D = sm + (s % kWStages) * kStage + ty * kWPitch;
+        const float* X = sm + (s % kWStages) * kStage + (TM + tx) * kWPitch;
+#pragma unroll 2
+        for (int q = grp; q < kWS / 4; q += GROUPS) {
+            ulonglong2 x[4];
+#pragma unroll
+            for (int w = 0; w < 4; ++w)
+                x[w] = *reinterpret_cast<const ulonglong2*>(X + w * TX * kWPitch + 4 * q);
+#pragma unroll
+            for (int u = 0; u < RU; ++u) {
+                const ulonglong2 d =
+                    *reinterpret_cast<const ulonglong2*>(D + u * TY * kWPitch + 4 * q);
+#pragma unroll
+                for (int w = 0; w < 4; ++w)
+                    acc[u][w] = fma2(d.y, x[w].y, fma2(d.x, x[w].x, acc[u][w]));
+            }
+        }
+    }
+    simt::cp_async_wait<0>();
+    __syncthreads();
+    // group sums, then the chunk's partial in group order
+#pragma unroll
+    for (int u = 0; u < RU; ++u)
 #pragma unroll
         for (int w = 0; w < 4; ++w) {
-            const uint32_t k = n0 + tx * 4 + w;
-            if (k < j.N) out[(size_t)m * j.ldw + k] = acc[u][w];
+            float e, o;
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(e), "=f"(o) : "l"(acc[u][w]));
+            sm[grp * TM * TN + (ty + u * TY) * TN + tx + w * TX] = e + o;
         }
+    __syncthreads();
+    for (int e = tid; e < TM * TN; e += kWThr) {
+        const uint32_t m = e / TN, k = e % TN;
+        if (m >= j.M || k >= j.store_n) continue;
+        float t = 0.f;
+#pragma unroll
+        for (int g = 0; g < GROUPS; ++g) t += sm[g * TM * TN + e];
+        out[(size_t)m * j.ldw + k] = t;
     }
 }
 
-// gradients = sum of the chunk partials in chunk order; entries no job writes (zero input
-// lanes) are zero in every partial, set once at creation
-__global__ void k_wreduce(const float* partial, uint32_t chunks, uint32_t total, float* grad,
-                          float scale) {
-    for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
-        float s = 0.f;
-        for (uint32_t c = 0; c < chunks; ++c) s += partial[(size_t)c * total + e];
+// the tile shapes: rows (delta) x columns (activation) of an output tile
+struct WShape {
+    uint32_t tm, tn;
+};
+constexpr WShape kWShapes[] = {{64, 64}, {32, 32}, {64, 16}, {32, 16}, {8, 64}, {8, 32}};
+
+// Bound by the FP32 FMA pipe for the square tiles and by HBM for the narrow output layers (both
+// operands are read once per output tile). 64 x 64 tiles of 8 x 4 outputs per thread read 12
+// 16-byte words per 128 FMAs; two CTAs per SM. The tile follows the layer (32 x 32 for the shipped
+// network, 8 rows for the output layers), so little work is done for padding. Measured: 64 x 2,
+// 262,144 samples 272 us, where 16 outputs per thread fed by scalar shared-memory reads, one
+// stage deep, took 937 us; shipped network, 50,021 samples 44 us against 419 us (25 chunks of
+// 2,048 left the chip idle).
+__global__ void __launch_bounds__(kWThr, 2) k_wgrad(const __grid_constant__ WGradArgs a) {
+    extern __shared__ float4 smem4[];
+    float* sm = reinterpret_cast<float*>(smem4);
+    const WJob& j = a.job[blockIdx.y];
+    const uint32_t i0 = blockIdx.x * a.chunk;
+    const uint32_t i1 = min(a.n, i0 + a.chunk);
+    float* out = a.partial + (size_t)blockIdx.x * a.total + j.out;
+    switch (j.shape) {
+        case 0: wgrad_tile<8, 8, 16>(a, j, sm, i0, i1, out); break;
+        case 1: wgrad_tile<4, 8, 8>(a, j, sm, i0, i1, out); break;
+        case 2: wgrad_tile<8, 8, 4>(a, j, sm, i0, i1, out); break;
+        case 3: wgrad_tile<4, 8, 4>(a, j, sm, i0, i1, out); break;
+        case 4: wgrad_tile<4, 2, 16>(a, j, sm, i0, i1, out); break;
+        default: wgrad_tile<4, 2, 8>(a, j, sm, i0, i1, out); break;
+    }
+}
+
+// samples per weight-gradient chunk of an n-sample step: 256 chunks (times the layers: several
+// waves of the grid, so that the last one costs little), and at least 256 samples to each, four
+// stages, so that a chunk's start-up and its partial stay small beside it
+uint32_t wgrad_chunk(uint64_t n) {
+    uint64_t c = (n + 255) / 256;
+    c = (c + kWS - 1) / kWS * kWS;
+    return (uint32_t)(c < 256 ? 256 : c);
+}
+// chunk partials that steps of up to n samples need
+uint64_t wgrad_chunks_max(uint64_t n) {
+    const uint64_t c = (n + 255) / 256;
+    return c < 256 ? c : 256;
+}
+
+// the output tiles of one layer (M outputs x N stored inputs of width ldw) as jobs
+int add_layer_jobs(WJob* job, uint32_t d_row, uint32_t a_row, uint32_t M, uint32_t N,
+                   uint32_t ldw, uint32_t out) {
+    uint32_t shape = 0;
+    if (M <= 8) shape = ldw >= 64 ? 4 : 5;
+    else if (ldw <= 16) shape = M >= 64 ? 2 : 3;
+    else shape = M >= 64 ? 0 : 1;
+    const WShape t = kWShapes[shape];
+    int k = 0;
+    for (uint32_t m = 0; m < M; m += t.tm)
+        for (uint32_t n = 0; n < ldw; n += t.tn) {
+            const uint32_t mv = M - m < t.tm ? M - m : t.tm, nv = N - n < t.tn ? N - n : t.tn;
+            const uint32_t sv = ldw - n < t.tn ? ldw - n : t.tn;
+            job[k++] = WJob{d_row + m, a_row + n, mv, nv, sv, ldw, out + m * ldw + n, shape};
+        }
+    return k;
+}
+
+// gradients = sum of the chunk partials of [chunks][stride] for the first `count` entries, in a
+// fixed order: eight slices of consecutive chunks, each in chunk order, then the slices in order.
+// Latency-bound (a few MB from L2): one serial sum per entry over 128 partials of the 64 x 2
+// networks took 11.0 us; eight slices over 256 partials take 5.2 us.
+constexpr int kRedSlices = 8;
+__global__ void __launch_bounds__(32 * kRedSlices) k_wreduce(const float* partial, uint32_t chunks,
+                                                             uint32_t stride, uint32_t count,
+                                                             float* grad, float scale) {
+    __shared__ float red[kRedSlices][32];
+    const uint32_t lane = threadIdx.x & 31u, sl = threadIdx.x >> 5;
+    const uint32_t e = blockIdx.x * 32u + lane;
+    const uint32_t per = (chunks + kRedSlices - 1) / kRedSlices;
+    const uint32_t c0 = sl * per, c1 = min(chunks, c0 + per);
+    float s = 0.f;
+    if (e < count)
+#pragma unroll 8
+        for (uint32_t c = c0; c < c1; ++c) s += partial[(size_t)c * stride + e];
+    red[sl][lane] = s;
+    __syncthreads();
+    if (sl == 0 && e < count) {
+#pragma unroll
+        for (int k = 1; k < kRedSlices; ++k) s += red[k][lane];
         grad[e] = s * scale;
     }
 }
@@ -722,9 +863,10 @@ uint32_t ld_of(uint32_t n) { return (n + 127) / 128 * 128; }
 
 }  // namespace
 
-cudaError_t launch_wreduce(const float* partial, uint32_t chunks, uint32_t total, float* grad,
-                           float scale, cudaStream_t s) {
-    k_wreduce<<<(total + 255) / 256, 256, 0, s>>>(partial, chunks, total, grad, scale);
+cudaError_t launch_wreduce(const float* partial, uint32_t chunks, uint32_t stride, uint32_t count,
+                           float* grad, float scale, cudaStream_t s) {
+    k_wreduce<<<(count + 31) / 32, 32 * kRedSlices, 0, s>>>(partial, chunks, stride, count, grad,
+                                                            scale);
     return cudaGetLastError();
 }
 
@@ -796,7 +938,7 @@ size_t train_scratch_bytes(const nrrs_config& c, uint32_t n, int sm_count) {
                          c.statnet_width * c.statnet_width + 3ull * c.statnet_width +
                          16ull * c.rrsnet_width + (uint64_t)(c.rrsnet_hidden - 1) * c.rrsnet_width *
                          c.rrsnet_width + (uint64_t)c.rrsnet_width;
-    const uint64_t chunks = (n + kChunk - 1) / kChunk;
+    const uint64_t chunks = wgrad_chunks_max(n);
     return sizeof(float) * (uint64_t)L.rows * ld_of(n) + sizeof(double) * 4 * (uint64_t)sm_count * 16 +
            sizeof(float) * chunks * mlp + 1024;
 }
@@ -808,7 +950,8 @@ int train_step_impl(nrrs_ctx* ctx, const VertexPtrs& v, const float* target, uin
     const nrrs_config& c = ctx->cfg;
     const Layout L = layout_of(c);
     const uint32_t ld = ld_of(c.max_train);
-    const uint64_t chunks = (n + kChunk - 1) / kChunk;
+    const uint32_t chunk = wgrad_chunk(n);
+    const uint64_t chunks = (n + chunk - 1) / chunk;
     const uint64_t mlp = ctx->n_stat + ctx->n_rrs;
     uint8_t* base = reinterpret_cast<uint8_t*>(ctx->train_scratch);
     float* act = reinterpret_cast<float*>(base);
@@ -820,8 +963,6 @@ int train_step_impl(nrrs_ctx* ctx, const VertexPtrs& v, const float* target, uin
 
     // gradients of this step only
     e = cudaMemsetAsync(ctx->grads, 0, sizeof(float) * ctx->n_params, s);
-    if (e == cudaSuccess)
-        e = cudaMemsetAsync(partial, 0, sizeof(float) * chunks * mlp, s);
     if (e != cudaSuccess) {
         ctx->last_error = std::string("train memset: ") + cudaGetErrorString(e);
         return NRRS_ERR_CUDA;
@@ -869,43 +1010,47 @@ int train_step_impl(nrrs_ctx* ctx, const VertexPtrs& v, const float* target, uin
     w.act = act;
     w.ld = ld;
     w.n = n;
-    w.chunks = (uint32_t)chunks;
+    w.chunk = chunk;
     w.partial = partial;
     w.total = (uint32_t)mlp;
-    int nj = 0;
-    uint32_t off = 0;
     const uint32_t WS = c.statnet_width, HS = c.statnet_hidden;
     const uint32_t WR = c.rrsnet_width, HR = c.rrsnet_hidden;
     const bool ref = c.network == NRRS_NET_REFERENCE;
     const uint32_t sin = stat_in_of((int)WS), sout = stat_out_of((int)WS);
-    w.job[nj++] = WJob{L.r_dhs, L.r_x0, WS, ref ? (uint32_t)kRefStatIn : 56u, sin, off};
+    int nj = 0;
+    uint32_t off = 0;
+    nj += add_layer_jobs(w.job + nj, L.r_dhs, L.r_x0, WS, ref ? (uint32_t)kRefStatIn : 56u, sin, off);
     off += WS * sin;
     for (uint32_t h = 1; h < HS; ++h) {
-        w.job[nj++] = WJob{L.r_dhs + h * WS, L.r_hs + (h - 1) * WS, WS, WS, WS, off};
+        nj += add_layer_jobs(w.job + nj, L.r_dhs + h * WS, L.r_hs + (h - 1) * WS, WS, WS, WS, off);
         off += WS * WS;
     }
-    w.job[nj++] = WJob{L.r_dy, L.r_hs + (HS - 1) * WS, sout, WS, WS, off};
+    nj += add_layer_jobs(w.job + nj, L.r_dy, L.r_hs + (HS - 1) * WS, sout, WS, WS, off);
     off += sout * WS;
     if (train_rrs) {
-        w.job[nj++] = WJob{L.r_dhr, L.r_x1, WR, ref ? (uint32_t)kRefRrsLanes : 10u, kRrsIn, off};
+        nj += add_layer_jobs(w.job + nj, L.r_dhr, L.r_x1, WR, ref ? (uint32_t)kRefRrsLanes : 10u,
+                             kRrsIn, off);
         off += WR * kRrsIn;
         for (uint32_t h = 1; h < HR; ++h) {
-            w.job[nj++] = WJob{L.r_dhr + h * WR, L.r_hr + (h - 1) * WR, WR, WR, WR, off};
+            nj += add_layer_jobs(w.job + nj, L.r_dhr + h * WR, L.r_hr + (h - 1) * WR, WR, WR, WR, off);
             off += WR * WR;
         }
-        w.job[nj++] = WJob{L.r_draw, L.r_hr + (HR - 1) * WR, 1, WR, WR, off};
+        nj += add_layer_jobs(w.job + nj, L.r_draw, L.r_hr + (HR - 1) * WR, 1, WR, WR, off);
+        off += WR;
     }
-    w.njobs = nj;
-    const uint32_t tiles_y = ((128 + 63) / 64) * ((128 + 63) / 64);
-    {
+    e = cudaFuncSetAttribute(k_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWSmem);
+    if (e == cudaSuccess) {
         ProfScope ps(ctx, NRRS_KERNEL_TRAIN_WGRAD, s);
-        k_wgrad<<<dim3((unsigned)chunks, tiles_y, (unsigned)nj), 256, 0, s>>>(w);
+        k_wgrad<<<dim3((unsigned)chunks, (unsigned)nj), kWThr, kWSmem, s>>>(w);
+        e = cudaGetLastError();
     }
-    {
+    if (e == cudaSuccess) {
+        // the first `off` entries have partials; gradients of untrained layers stay zero
         ProfScope ps(ctx, NRRS_KERNEL_TRAIN_REDUCE, s);
-        e = launch_wreduce(partial, (uint32_t)chunks, (uint32_t)mlp, ctx->grads + ctx->n_table, 1.0f, s);
+        e = launch_wreduce(partial, (uint32_t)chunks, (uint32_t)mlp, off, ctx->grads + ctx->n_table,
+                           1.0f, s);
     }
-    if ((e = cudaGetLastError()) != cudaSuccess) {
+    if (e != cudaSuccess) {
         ctx->last_error = std::string("wgrad launch: ") + cudaGetErrorString(e);
         return NRRS_ERR_CUDA;
     }

@@ -864,8 +864,8 @@ size_t train_tc_scratch_bytes(const nrrs_config& c, uint32_t n, int sm_count) {
            sizeof(float) * 32ull * n + 1024;
 }
 
-cudaError_t launch_wreduce(const float* partial, uint32_t chunks, uint32_t total, float* grad,
-                           float scale, cudaStream_t s);
+cudaError_t launch_wreduce(const float* partial, uint32_t chunks, uint32_t stride, uint32_t count,
+                           float* grad, float scale, cudaStream_t s);
 int train_step_tc(nrrs_ctx* ctx, const VertexPtrs& v, const float* target, uint32_t n,
                   double* loss_dev, cudaStream_t s, bool apply, const LossWeights* lw) {
     const nrrs_config& c = ctx->cfg;
@@ -1071,7 +1071,8 @@ int train_step_tc(nrrs_ctx* ctx, const VertexPtrs& v, const float* target, uint3
     }
     if (e == cudaSuccess) {
         ProfScope ps(ctx, NRRS_KERNEL_TRAIN_REDUCE, s);
-        e = launch_wreduce(partial, (uint32_t)chunks, (uint32_t)mlp, ctx->grads + ctx->n_table,
+        e = launch_wreduce(partial, (uint32_t)chunks, (uint32_t)mlp, (uint32_t)mlp,
+                           ctx->grads + ctx->n_table,
                            1.0f / (float)n, s);
     }
     join();  // the table gradient is complete on s from here
