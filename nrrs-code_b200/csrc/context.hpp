@@ -39,7 +39,10 @@ struct nrrs_ctx {
     float* adam_v = nullptr;   // [n_params]
     uint64_t adam_t = 0;
 
-    __half* table_h = nullptr; // FP16 table copy (mixed precision)
+    // FP16 table copy (mixed precision): row r of the table is entry r + shift_h, so that the
+    // hashed levels start on a 32-byte sector (half_shift)
+    __half* table_h = nullptr;
+    uint32_t shift_h = 0;
     uint4* cells = nullptr;    // cell image of the FP16 table's dense levels (EncodeParams::cells)
     uint32_t n_cells = 0;
     // moving average of the weights (ema_decay > 0): the raw average, its debiased copy and the
@@ -117,6 +120,12 @@ struct ProfScope {
 }  // namespace nrrs
 
 namespace nrrs {
+// the level table of the FP16 table's layout
+inline EncodeParams half_enc(const nrrs_ctx* ctx) {
+    EncodeParams e = ctx->enc;
+    for (uint32_t l = 0; l < e.n_levels; ++l) e.lv[l].offset += ctx->shift_h;
+    return e;
+}
 // gradients of one step; with apply, the Adam update too
 // (lw: per-sample loss weights of nrrs_train_step_batch; NULL = plain means)
 int train_step_impl(nrrs_ctx* ctx, const VertexPtrs& v, const float* target, uint32_t n,

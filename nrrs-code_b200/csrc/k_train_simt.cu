@@ -701,7 +701,8 @@ int add_layer_jobs(WJob* job, uint32_t d_row, uint32_t a_row, uint32_t M, uint32
 // gradients = sum of the chunk partials of [chunks][stride] for the first `count` entries, in a
 // fixed order: eight slices of consecutive chunks, each in chunk order, then the slices in order.
 // Latency-bound (a few MB from L2): one serial sum per entry over 128 partials of the 64 x 2
-// networks took 11.0 us; eight slices over 256 partials take 5.2 us.
+// networks took 11.0 us; eight slices over 256 partials take 5.2 us. 128 x 3 networks (90,000
+// entries, 55 partials): 18.3 -> 12.6 us.
 constexpr int kRedSlices = 8;
 __global__ void __launch_bounds__(32 * kRedSlices) k_wreduce(const float* partial, uint32_t chunks,
                                                              uint32_t stride, uint32_t count,
@@ -713,8 +714,14 @@ __global__ void __launch_bounds__(32 * kRedSlices) k_wreduce(const float* partia
     const uint32_t c0 = sl * per, c1 = min(chunks, c0 + per);
     float s = 0.f;
     if (e < count)
-#pragma unroll 8
-        for (uint32_t c = c0; c < c1; ++c) s += partial[(size_t)c * stride + e];
+        for (uint32_t c = c0; c < c1; c += 8) {   // eight loads in flight, whatever the remainder
+            float v[8];
+#pragma unroll
+            for (uint32_t k = 0; k < 8; ++k)
+                v[k] = c + k < c1 ? partial[(size_t)(c + k) * stride + e] : 0.f;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) s += v[k];
+        }
     red[sl][lane] = s;
     __syncthreads();
     if (sl == 0 && e < count) {
@@ -774,7 +781,10 @@ __global__ void k_adam(const __grid_constant__ AdamArgs a) {
             uint2 u;
             u.x = *reinterpret_cast<uint32_t*>(&h0);
             u.y = *reinterpret_cast<uint32_t*>(&h1);
-            *reinterpret_cast<uint2*>(a.table_h + k) = u;
+            // 4-byte stores where the table's shift is an odd number of rows
+            uint32_t* d = reinterpret_cast<uint32_t*>(a.table_h + k);
+            if ((reinterpret_cast<uintptr_t>(d) & 7u) == 0) *reinterpret_cast<uint2*>(d) = u;
+            else d[0] = u.x, d[1] = u.y;
         } else if (a.table_h) {
             const float nv[4] = {nw.x, nw.y, nw.z, nw.w};
             for (int j = 0; j < 4; ++j)
@@ -880,7 +890,7 @@ cudaError_t launch_adam_step(nrrs_ctx* ctx, bool train_rrs, cudaStream_t s, floa
     ad.gscale = scale;
     ad.m = ctx->adam_m;
     ad.v = ctx->adam_v;
-    ad.table_h = ctx->table_h;
+    ad.table_h = ctx->table_h ? ctx->table_h + 2 * ctx->shift_h : nullptr;
     ad.n_table = ctx->n_table;
     ad.first = 0;
     ad.count = ctx->n_table + ctx->n_stat + (train_rrs ? ctx->n_rrs : 0);
@@ -900,7 +910,7 @@ cudaError_t launch_adam_step(nrrs_ctx* ctx, bool train_rrs, cudaStream_t s, floa
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess && ctx->cells) {
         ProfScope ps(ctx, NRRS_KERNEL_CELL_IMAGE, s);
-        e = launch_cell_image(ctx->table_h, ctx->enc, ctx->cells, ctx->n_cells, ctx->sm_count, s);
+        e = launch_cell_image(ctx->table_h, half_enc(ctx), ctx->cells, ctx->n_cells, ctx->sm_count, s);
     }
     if (e != cudaSuccess || !ctx->ema) return e;
     // the moving average of every parameter and the inference table derived from it
@@ -909,7 +919,7 @@ cudaError_t launch_adam_step(nrrs_ctx* ctx, bool train_rrs, cudaStream_t s, floa
     ea.p = ctx->params;
     ea.e = ctx->ema;
     ea.pi = ctx->params_inf;
-    ea.table_h = ctx->table_h_inf;
+    ea.table_h = ctx->table_h_inf ? ctx->table_h_inf + 2 * ctx->shift_h : nullptr;
     ea.n_table = ctx->n_table;
     ea.count = ctx->n_params;
     ea.d = c.ema_decay;
@@ -922,7 +932,7 @@ cudaError_t launch_adam_step(nrrs_ctx* ctx, bool train_rrs, cudaStream_t s, floa
     e = cudaGetLastError();
     if (e != cudaSuccess || !ctx->cells_inf) return e;
     ProfScope ps(ctx, NRRS_KERNEL_CELL_IMAGE, s);
-    return launch_cell_image(ctx->table_h_inf, ctx->enc, ctx->cells_inf, ctx->n_cells,
+    return launch_cell_image(ctx->table_h_inf, half_enc(ctx), ctx->cells_inf, ctx->n_cells,
                              ctx->sm_count, s);
 }
 

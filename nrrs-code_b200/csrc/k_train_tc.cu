@@ -45,6 +45,7 @@ struct TcTrainArgs {
     float loss_clamp, cost_offset, inv_n;
     int32_t train_rrs;
     const __half* table_h;
+    uint32_t shift_h;       // entry of table_h that holds row 0
     float* table_grad;
     const uint8_t* tpack;   // training image (forward layers)
     uint32_t s_bytes;       // StatNet image bytes (at tpack + 0)
@@ -235,7 +236,8 @@ __global__ void __launch_bounds__(128 * WGS, 1) k_ttc_stat(const __grid_constant
                 float f[8];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const LevelDev L = a.enc.lv[lq * 4 + j];
+                    LevelDev L = a.enc.lv[lq * 4 + j];
+                    L.offset += a.shift_h;
                     const CellCoord c = cell_of(p, L.res);
                     const float2 fv =
                         level_features_h<(W < 128)>(table, a.enc.cells, L, a.enc.hash_mask, c);
@@ -916,6 +918,7 @@ int train_step_tc(nrrs_ctx* ctx, const VertexPtrs& v, const float* target, uint3
     a.inv_n = 1.0f / (float)n;
     a.train_rrs = train_rrs;
     a.table_h = ctx->table_h;
+    a.shift_h = ctx->shift_h;
     a.table_grad = ctx->grads;
     a.tpack = reinterpret_cast<const uint8_t*>(ctx->tpack);
     const int W = c.statnet_width, H = c.statnet_hidden;
@@ -935,7 +938,7 @@ int train_step_tc(nrrs_ctx* ctx, const VertexPtrs& v, const float* target, uint3
     if (split) {
         // hash columns of the x0 tiles, level-major (FP16, the StatNet training precision)
         EncodeLvArgs ea{};
-        ea.enc = ctx->enc;
+        ea.enc = half_enc(ctx);
         ea.segs.n = 1;
         ea.segs.s[0].offset = 0;
         ea.segs.s[0].count = n;

@@ -146,8 +146,11 @@ __global__ void k_cell_image(const uint32_t* __restrict__ rows,
         for (int k = 0; k < 8; ++k)
             t[k] = rows[grid_row(L, e.hash_mask, x + (k & 1), y + ((k >> 1) & 1),
                                  z + ((k >> 2) & 1))];
-        cells[2 * (size_t)g] = make_uint4(t[0], t[1], t[2], t[3]);
-        cells[2 * (size_t)g + 1] = make_uint4(t[4], t[5], t[6], t[7]);
+        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(
+                         cells + 2 * (size_t)g),
+                     "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]), "r"(t[4]), "r"(t[5]), "r"(t[6]),
+                     "r"(t[7])
+                     : "memory");
     }
 }
 

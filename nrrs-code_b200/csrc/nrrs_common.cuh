@@ -293,7 +293,8 @@ __device__ __forceinline__ uint32_t quad_pick(const uint4& q, uint32_t e) {
 // The 8 corner entries (FP16 pairs, as raw 32-bit words) of a cell, in corner order. For each
 // (y, z) the aligned 16-byte quad holding corner x is loaded; corner x+1 comes from the same
 // quad when it lies there (dense rows are consecutive, and the hash multiplies x by 1, so x and
-// x+1 differ in the low bits: 3 times in 4) and from a predicated 4-byte load otherwise. That is
+// x+1 differ in the low bits: 3 times in 4, given that a hashed level starts on a quad, which the
+// FP16 table's shift sees to) and from a predicated 4-byte load otherwise. That is
 // about 5 L1 requests per level instead of 8 for the same values; the table carries 16 bytes of
 // padding for the last quad.
 // the 8 corner entries of cell c of dense level L from the cell image: one 32-byte load
