@@ -34,6 +34,7 @@ struct nrrs_ctx {
     uint64_t n_table = 0, n_stat = 0, n_rrs = 0, n_params = 0;
 
     float* params = nullptr;   // FP32 master [n_params]
+    uint32_t params_pad = 0;   // floats of the params and params_inf allocations before them
     float* grads = nullptr;    // [n_params]
     float* adam_m = nullptr;   // [n_params]
     float* adam_v = nullptr;   // [n_params]
@@ -87,6 +88,8 @@ struct nrrs_ctx {
     int train_split = 1;         // training mode of the tcgen05 path: 0 fused, 1 split
     uint8_t* enc_tiles = nullptr;  // split mode: hash-feature tiles (kEncTileBytes each)
     uint32_t enc_tiles_cap = 0;
+    float* feat = nullptr;         // FP32 path: hash features of one inference pass
+    uint32_t feat_tiles = 0;       // its tiles
     uint8_t* x1_tiles = nullptr;   // split mode 2: RRSNet input tiles (kX1TileBytes each)
     nrrs::Profiler prof;
     std::string last_error;
@@ -134,6 +137,16 @@ int train_step_impl(nrrs_ctx* ctx, const VertexPtrs& v, const float* target, uin
 // batch sums of the loss weights into out[3] (sum s, sum w, mean pixel error)
 cudaError_t launch_loss_sums(const LossWeights& w, uint32_t n, const float* error_sum,
                              uint32_t n_pixels, double* out, cudaStream_t s);
+// The table gradient of an n-sample step from its lane gradients, added to zeroed slices of
+// ctx->grads level group by level group (k_train_tc.cu). Component c of level l of sample i is
+// dxs[l * level_stride + i * sample_stride + c * comp_stride]; it is multiplied by scale.
+struct LaneGrads {
+    const float* dxs;
+    size_t level_stride, sample_stride, comp_stride;
+    float scale;
+};
+cudaError_t launch_scatter_table(nrrs_ctx* ctx, const float* pos, uint32_t n, const LaneGrads& g,
+                                 cudaStream_t s);
 // Adam on ctx->grads scaled by `scale` (copied in from grads_dev first when it is not ctx->grads)
 cudaError_t launch_adam_step(nrrs_ctx* ctx, bool train_rrs, cudaStream_t s, float scale = 1.0f);
 size_t train_scratch_bytes(const nrrs_config& cfg, uint32_t n, int sm_count);

@@ -1,5 +1,6 @@
-// k_encode.cu -- level-major hash-grid encoding into feature tiles (sm_100a), the first kernel
-// of the split inference mode.
+// k_encode.cu -- level-major hash-grid encoding (sm_100a): into feature tiles, the first kernel of
+// the split inference mode and of the mixed training step, and into FP32 features, the first kernel
+// of the FP32 path.
 //
 // With a table larger than L2 (16 levels of 2^22 FP16 pairs: 178 MB), the fused inference
 // kernel gathers each vertex's 128 corners from all 16 levels at once, so the lines in flight
@@ -17,7 +18,7 @@
 // The per-level arithmetic is that of the fused kernel (levels_features_h), so the features and
 // everything downstream are bit-identical between the two modes. The encoding is the
 // reference's tcnn HashGrid (common/configs/nrrs/nrrs/2net-simple.json:46).
-#include "kernels.hpp"
+#include "simt_gemm.cuh"
 #include "tc_tile.cuh"
 
 namespace nrrs {
@@ -54,7 +55,48 @@ __global__ void __launch_bounds__(kTile) k_encode_levels(const __grid_constant__
     }
 }
 
+// The FP32 path's encoding, one work item per (4 levels, tile), level-major: a kernel of its own
+// keeps 32 warps per SM on the gathers, where the fused FP32 kernels' 16 waited for them
+// (64 x 2 networks, 262,144 samples: 89 us for the
+// encoding, 330 us inside the training kernel).
+__global__ void __launch_bounds__(kTile) k_encode_f32(const __grid_constant__ EncodeF32Args a) {
+    const uint32_t tiles = a.tile_end - a.tile_begin;
+    const uint32_t items = a.enc.n_levels / 4 * tiles;
+    const SegmentTable& S = seg_table(a.segs);
+    const float2* table = reinterpret_cast<const float2*>(a.table);
+    const int m = threadIdx.x;
+    for (uint32_t w = blockIdx.x; w < items; w += gridDim.x) {
+        const uint32_t q = w / tiles, tt = w - q * tiles, t = a.tile_begin + tt;
+        if (t >= S.total_tiles) continue;
+        const Segment& sg = S.s[find_segment(S, t)];
+        const uint32_t i = sg.offset + (t - sg.tile_start) * kTile + m;
+        const bool valid = i < sg.offset + sg.count;
+        float* out = a.out + tt * a.tile_stride + 8 * q * a.lane_stride + m;
+        float p[3] = {0.f, 0.f, 0.f};
+        if (valid) norm_pos(a.enc, a.pos, i, p);
+#pragma unroll 2
+        for (int j = 0; j < 4; ++j) {
+            float2 f = make_float2(0.f, 0.f);
+            if (valid) {
+                const LevelDev L = a.enc.lv[4 * q + j];
+                f = simt::level_features_f(table, L, a.enc.hash_mask, cell_of(p, L.res));
+            }
+            out[(2 * j) * a.lane_stride] = f.x;
+            out[(2 * j + 1) * a.lane_stride] = f.y;
+        }
+    }
+}
+
 }  // namespace
+
+cudaError_t launch_encode_f32(const EncodeF32Args& a, int sm_count, cudaStream_t s) {
+    const uint32_t items = a.enc.n_levels / 4 * (a.tile_end - a.tile_begin);
+    if (items == 0) return cudaSuccess;
+    const uint32_t most =
+        (uint32_t)(sm_count * resident_ctas((const void*)k_encode_f32, kTile, 0, 16));
+    k_encode_f32<<<items < most ? items : most, kTile, 0, s>>>(a);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_encode_levels(const EncodeLvArgs& a, bool bf, int sm_count, cudaStream_t s) {
     const uint32_t items = 4u * a.segs.total_tiles;

@@ -7,107 +7,57 @@
 // nrrs_generate_inference_data_from_0to1 (train.cu:41-112) and the "Gen RRS Number" lambda
 // (integrator.cpp:1184-1298), so the AoS round trips of the reference disappear.
 //
-// A CTA of 128 threads works on 64 vertices at a time (half of a 128-vertex tile of the segment
-// table). Their activations live in one shared-memory tile, K-major ([k][64 vertices + 4 pad]).
-// Every hidden layer is a register-tiled FP32 GEMM: each thread owns an 8 x (W/16) block of outputs
-// (8 vertices x 8 or 4 neurons), and per k it reads 8 activations and 8 (or 4) weights as
-// float4 and issues 64 (or 32) FMAs. The layer's transposed weights ([in][out]) come from L2 in
-// 32-row chunks, double-buffered with cp.async while the previous chunk is consumed. Every output
-// is accumulated as fmaf(w_k, x_k, acc) over k ascending, the same sequence for any launch shape.
-// The narrow layers (3 and 1 outputs), the glue, the factor and the exact-sum term run one thread
-// per vertex on that vertex's column of the tile.
+// A CTA works on 64 vertices at a time (half of a 128-vertex tile of the segment table) with 64
+// threads (128 for the 128-wide networks). Their activations live in one shared-memory tile;
+// every hidden layer is a register-tiled FP32 GEMM in place on it (simt_gemm.cuh). The encoding,
+// the narrow layers (3 and 1 outputs), the glue, the factor and the exact-sum term run one thread
+// per vertex on that vertex's column of the tile (two for the encoding of the 128-wide networks).
+// Every output is accumulated as fmaf(w_k, x_k, acc) over k ascending, the same sequence for any
+// launch shape.
+// The hash features come from the encoding kernel (k_encode.cu), in passes of at most 1,048,576
+// vertices. 64 x 2 networks, 65,536 vertices: 47 us and 24 us of encoding, where one kernel that
+// gathered for itself took 106 us with 128 threads per CTA (8 x 4 outputs each, 1.15 waves) and 90
+// with 64; the FMA pipe's floor is 24 us.
 #include "simt_gemm.cuh"
 
 namespace nrrs {
 
 namespace {
 
-using simt::kLd;
-using simt::kThr;
+using simt::at;
 using simt::kTM;
 
 template <int W>
 struct FpShape {
-    static constexpr int kRows = simt::imax(stat_in_of(W), W);     // rows of the activation tile
-    static constexpr int kActFloats = kRows * kLd;
+    static constexpr int kThr = simt::threads_of(W);
+    static constexpr int kActFloats = simt::imax(stat_in_of(W), W) * kTM;
     static constexpr int kChunkFloats = simt::kKC * W;
     static constexpr size_t kSmem = sizeof(float) * (kActFloats + 2 * kChunkFloats);
 };
 
 // out[n][m] = act(sum_k wt[k][n] act[k][m]) for k < k_eff, in place on the activation tile, with
-// ReLU (the workload's network) or LeakyReLU (the reference network, W = 32); wt is [k_rows][W]
-// in global memory; rows k_eff .. k_rows-1 are loaded but multiply zeros.
+// ReLU (the workload's network) or LeakyReLU (the reference network, W = 32); wt is [in][W] in
+// global memory (input lanes from k_eff on are zero)
 template <int W>
-__device__ __forceinline__ void hidden_layer(const float* __restrict__ wt, int k_rows, int k_eff,
-                                             float* act, float* wch, int tid) {
-    simt::tile_gemm<W>(wt, k_rows, k_eff, act, wch, tid, [&](int n, int m0, const float* v) {
-        float r[8];
+__device__ __forceinline__ void hidden_layer(const float* __restrict__ wt, int k_eff, float* act,
+                                             float* wch, int tid) {
+    simt::tile_gemm<W, FpShape<W>::kThr>(
+        wt, W, k_eff, act, wch, tid, [&](int, int n, int m0, const float* v) {
+            float r[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) r[i] = W == 32 ? leaky(v[i]) : fmaxf(v[i], 0.f);
-        simt::tile_store8(act, n, m0, r);
-    });
-}
-
-// the network's narrow output layer for vertex column m: y[o] = sum_k wt[k][o] act[k][m], with
-// wt [W][OUT rounded up to 4]
-template <int W, int OUT>
-__device__ __forceinline__ void output_layer(const float* __restrict__ wt, const float* act, int m,
-                                             float* y) {
-    constexpr int OP = (OUT + 3) / 4 * 4;
-    float acc[OUT];
-#pragma unroll
-    for (int o = 0; o < OUT; ++o) acc[o] = 0.f;
-#pragma unroll 4
-    for (int k = 0; k < W; ++k) {
-        const float x = act[k * kLd + m];
-#pragma unroll
-        for (int q = 0; q < OP / 4; ++q) {
-            const float4 w = __ldg(reinterpret_cast<const float4*>(wt + OP * k + 4 * q));
-            const float wv[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-                if (4 * q + e < OUT) acc[4 * q + e] = fmaf(wv[e], x, acc[4 * q + e]);
-        }
-    }
-#pragma unroll
-    for (int o = 0; o < OUT; ++o) y[o] = acc[o];
-}
-
-// hash-grid levels l0 .. l0+NL-1 of vertex i into its column of the tile (FP32 table)
-template <int NL = 8>
-__device__ __forceinline__ void encode_levels8(const InferArgs& a, const float* p, int l0, float* act,
-                                               int m) {
-    const float2* table = reinterpret_cast<const float2*>(a.table);
-#pragma unroll 2
-    for (int l = l0; l < l0 + NL; ++l) {
-        const LevelDev L = a.enc.lv[l];
-        const CellCoord c = cell_of(p, L.res);
-        uint32_t rows[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-            rows[k] = grid_row(L, a.enc.hash_mask, c.ix + (k & 1), c.iy + ((k >> 1) & 1),
-                               c.iz + ((k >> 2) & 1));
-        float2 t[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) t[k] = __ldg(table + rows[k]);
-        float f0 = 0.f, f1 = 0.f;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const float w = corner_weight(c, k);
-            f0 += w * t[k].x;
-            f1 += w * t[k].y;
-        }
-        act[(2 * l) * kLd + m] = f0;
-        act[(2 * l + 1) * kLd + m] = f1;
-    }
+            for (int i = 0; i < 8; ++i) r[i] = W == 32 ? leaky(v[i]) : fmaxf(v[i], 0.f);
+            simt::tile_store8(act, n, m0, r);
+        });
 }
 
 template <int WS, int HS, int WR, int HR>
-__global__ void __launch_bounds__(kThr) k_infer_fp32(const __grid_constant__ InferArgs a) {
+__global__ void __launch_bounds__(FpShape<WS>::kThr, WS == 128 ? 4 : 8)
+    k_infer_fp32(const __grid_constant__ InferArgs a) {
     static_assert(WS == WR, "one tile shape for both networks");
     constexpr bool REF = WS == 32;             // the reference's shipped network
     constexpr int SIN = stat_in_of(WS), SOUT = stat_out_of(WS);
     using S = FpShape<WS>;
+    constexpr int TPS = S::kThr / kTM;         // threads per vertex of the encoding
     extern __shared__ float4 smem4[];
     float* act = reinterpret_cast<float*>(smem4);
     float* wch = act + S::kActFloats;
@@ -115,7 +65,8 @@ __global__ void __launch_bounds__(kThr) k_infer_fp32(const __grid_constant__ Inf
     const int m = tid & (kTM - 1);
     const bool lead = tid < kTM;               // the thread that owns vertex column m
     const SegmentTable& ST = seg_table(a.segs);
-    const uint32_t items = 2u * ST.total_tiles;
+    const uint32_t tile_end = min(a.tile_end, ST.total_tiles);
+    const uint32_t items = tile_end > a.tile_begin ? 2u * (tile_end - a.tile_begin) : 0u;
     // transposed layer images: [in][out] (outputs padded to 4), StatNet then RRSNet
     const float* s0 = a.wt_stat;
     const float* s_out = s0 + (size_t)SIN * WS + (size_t)(HS - 1) * WS * WS;
@@ -124,76 +75,73 @@ __global__ void __launch_bounds__(kThr) k_infer_fp32(const __grid_constant__ Inf
 
 #pragma unroll 1
     for (uint32_t u = blockIdx.x; u < items; u += gridDim.x) {
-        const uint32_t t = u >> 1;
+        const uint32_t t = a.tile_begin + (u >> 1);
         const int si = find_segment(ST, t);
         const Segment& sg = ST.s[si];
         const uint32_t i = sg.offset + (t - sg.tile_start) * kTile + (u & 1u) * kTM + m;
         const bool valid = i < sg.offset + sg.count;
         __syncthreads();   // the previous item's column reads are over
-        // encoding: two threads per vertex (levels 0-7 + SH, levels 8-15 + misc lanes; the
-        // reference network: levels 0-3 + direction blobs, levels 4-7 + roughness blob)
-        if (REF) {
-            if (valid) {
-                float p[3];
-                norm_pos(a.enc, a.v.pos, i, p);
-                encode_levels8<4>(a, p, lead ? 0 : 4, act, m);
+        // the hash features from the encoding kernel, the other input lanes here (one thread per
+        // vertex, or two)
+        const bool lo = TPS == 1 || lead, hi = TPS == 1 || !lead;
+        constexpr int HL = 2 * (REF ? kRefLevels : kMaxLevels);
+        simt::load_rows<HL, S::kThr>(a.feat + (size_t)(t - a.tile_begin) * kF32TileFloats +
+                                         (u & 1u) * kTM,
+                                     kTile, act, tid);
+        simt::cp_async_commit();
+        if (valid) {
+            if (REF) {
                 float blob[16];
                 ref_blob_lanes(a.v, i, blob);
 #pragma unroll
-                for (int k = 0; k < 8; ++k)
-                    act[(16 + (lead ? 0 : 8) + k) * kLd + m] = lead ? blob[k] : blob[8 + k];
+                for (int k = 0; k < 16; ++k)
+                    if (k < 8 ? lo : hi) act[at(HL + k, m)] = blob[k];
             } else {
-                for (int k = lead ? 0 : 16; k < (lead ? 16 : 32); ++k) act[k * kLd + m] = 0.f;
-            }
-        } else if (valid) {
-            float p[3];
-            norm_pos(a.enc, a.v.pos, i, p);
-            if (lead) {
-                encode_levels8(a, p, 0, act, m);
-                float sh[16];
-                const size_t i3 = 3 * (size_t)i;
-                sh16(a.v.wi[i3], a.v.wi[i3 + 1], a.v.wi[i3 + 2], sh);
+                if (lo) {
+                    float sh[16];
+                    const size_t i3 = 3 * (size_t)i;
+                    sh16(a.v.wi[i3], a.v.wi[i3 + 1], a.v.wi[i3 + 2], sh);
 #pragma unroll
-                for (int k = 0; k < 16; ++k) act[(32 + k) * kLd + m] = sh[k];
-            } else {
-                encode_levels8(a, p, 8, act, m);
-                float misc[16];
-                misc_lanes(a.v, i, misc);
+                    for (int k = 0; k < 16; ++k) act[at(32 + k, m)] = sh[k];
+                }
+                if (hi) {
+                    float misc[16];
+                    misc_lanes(a.v, i, misc);
 #pragma unroll
-                for (int k = 0; k < 8; ++k) act[(48 + k) * kLd + m] = misc[k];
+                    for (int k = 0; k < 8; ++k) act[at(48 + k, m)] = misc[k];
+                }
             }
         } else {
-            for (int k = lead ? 0 : 28; k < (lead ? 28 : 56); ++k) act[k * kLd + m] = 0.f;
+            constexpr int NO = REF ? 16 : 24;    // non-hash lanes; `hi` owns the last 8
+            for (int k = lo ? 0 : NO - 8; k < (hi ? NO : NO - 8); ++k) act[at(HL + k, m)] = 0.f;
         }
         VertexAux aux{};
         if (lead && valid) aux = load_aux(a.v, i);
         // StatNet: 56 live input lanes (48..55 misc, 56..63 zero); the reference network's 32
-        hidden_layer<WS>(s0, SIN, REF ? 32 : 56, act, wch, tid);
+        hidden_layer<WS>(s0, REF ? 32 : 56, act, wch, tid);
 #pragma unroll 1
         for (int h = 1; h < HS; ++h)
-            hidden_layer<WS>(s0 + (size_t)SIN * WS + (size_t)(h - 1) * WS * WS, WS, WS, act,
-                             wch, tid);
+            hidden_layer<WS>(s0 + (size_t)SIN * WS + (size_t)(h - 1) * WS * WS, WS, act, wch, tid);
         float y[SOUT];
 #pragma unroll
         for (int k = 0; k < SOUT; ++k) y[k] = 0.f;
         if (lead) {
-            output_layer<WS, SOUT>(s_out, act, m, y);
+            simt::narrow_out<WS, SOUT>(s_out, act, m, y);
             // glue: the RRSNet input in this vertex's column (10 live lanes; the reference's 12)
             float x1[16];
             if (REF) glue16_ref_aux(y, aux, x1);
             else glue16_aux(a.fp, y, aux, x1);
 #pragma unroll
-            for (int k = 0; k < (REF ? kRefRrsLanes : 10); ++k) act[k * kLd + m] = x1[k];
+            for (int k = 0; k < (REF ? kRefRrsLanes : 10); ++k) act[at(k, m)] = x1[k];
         }
-        hidden_layer<WR>(r0, kRrsIn, REF ? kRefRrsLanes : 10, act, wch, tid);
+        hidden_layer<WR>(r0, REF ? kRefRrsLanes : 10, act, wch, tid);
 #pragma unroll 1
         for (int h = 1; h < HR; ++h)
-            hidden_layer<WR>(r0 + (size_t)kRrsIn * WR + (size_t)(h - 1) * WR * WR, WR, WR, act,
-                             wch, tid);
+            hidden_layer<WR>(r0 + (size_t)kRrsIn * WR + (size_t)(h - 1) * WR * WR, WR, act, wch, tid);
         long long term = 0;
         if (lead && valid) {
             float raw;
-            output_layer<WR, 1>(r_out, act, m, &raw);
+            simt::narrow_out<WR, 1>(r_out, act, m, &raw);
             const float rrs = rrs_factor_aux<REF>(a.fp, y, raw, aux);
             if (a.stats) {
 #pragma unroll
@@ -218,14 +166,14 @@ cudaError_t launch_cfg(const InferArgs& a, int sm_count, int ctas_per_sm, cudaSt
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)S::kSmem);
     if (e != cudaSuccess) return e;
-    int per_sm = resident_ctas((const void*)kern, kThr, S::kSmem, 32);
+    int per_sm = resident_ctas((const void*)kern, S::kThr, S::kSmem, 32);
     if (ctas_per_sm > 0 && ctas_per_sm < per_sm) per_sm = ctas_per_sm;
-    const uint32_t items = 2u * a.segs.total_tiles;
+    const uint32_t items = 2u * (a.tile_end - a.tile_begin);
     unsigned grid = (unsigned)(sm_count * per_sm);
     if (grid > items) grid = items;
     if (grid == 0) return cudaSuccess;
     g_last_grid = (int)grid;
-    kern<<<grid, kThr, S::kSmem, s>>>(a);
+    kern<<<grid, S::kThr, S::kSmem, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -251,7 +199,7 @@ int max_ctas_fp32() {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::kSmem) !=
         cudaSuccess)
         return 0;
-    return resident_ctas((const void*)kern, kThr, S::kSmem, 32);
+    return resident_ctas((const void*)kern, S::kThr, S::kSmem, 32);
 }
 
 int infer_max_ctas_fp32(int ws, int hs) {

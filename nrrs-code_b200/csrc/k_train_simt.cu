@@ -10,11 +10,12 @@
 //   RRSNet inputs come from the detached StatNet forward of the same step (the reference trains
 //   the networks separately and builds RRSNet's input after StatNet's step, train.cu:155-240).
 //
-// Pipeline (all on the caller's stream, no host synchronisation):
-//   k_train_stat  per sample: encode, StatNet forward, loss gradient, backward to the input,
-//                 hash-grid scatter-add (FP32 atomics), glue; RRSNet forward for the batch sums
-//                 V and C (FP64 per-CTA partials). Activations and deltas go to feature-major
-//                 scratch for the weight gradients.
+// Pipeline (forked from and joined into the caller's stream, no host synchronisation):
+//   k_encode_f32  hash features of the batch, level-major (k_encode.cu).
+//   k_train_stat  per sample: StatNet forward, loss gradient, backward to the hash lanes, glue;
+//                 RRSNet forward for the batch sums V and C (FP64 per-CTA partials). Activations
+//                 and deltas go to feature-major scratch for the weight gradients.
+//   k_scatter_levels  the lane gradients into the table (FP32 reductions, k_train_tc.cu), beside
 //   k_train_rrs   per sample: RRSNet forward and backward with the final V and C.
 //   k_wgrad       dW = sum_i delta_i (x) a_i for every layer, split over sample chunks.
 //   k_wreduce     chunk partials -> gradients, in fixed order (deterministic).
@@ -26,25 +27,21 @@ namespace nrrs {
 
 namespace {
 
-constexpr int kTT = 128;           // threads per CTA of the training kernels
 
 struct TrainArgs {
     VertexPtrs v;
     const float* target;
     uint32_t n;
     uint32_t ld;                   // row stride of the feature-major scratch
-    EncodeParams enc;
     FactorParams fp;
     float loss_clamp, cost_offset;
     int32_t train_rrs;
-    const float* table;
-    float* table_grad;
     const float* wt_stat;          // transposed [in][out4] (forward)
     const float* wt_rrs;
     const float* w_stat;           // row-major master [out][in] (backward)
     const float* w_rrs;
     float* act;                    // feature-major scratch
-    uint32_t r_x0, r_hs, r_dhs, r_dy, r_x1, r_hr, r_dhr, r_draw;
+    uint32_t r_x0, r_hs, r_dhs, r_dx, r_dy, r_x1, r_hr, r_dhr, r_draw;
     double* part;                  // [grid][4]: loss_S sum, V sum, C sum, R sum
     uint32_t part_n;               // CTAs of k_train_stat
     double* loss_out;              // [2]
@@ -60,7 +57,7 @@ __device__ __forceinline__ double block_sum_d(double v, double* red) {
     __syncthreads();
     double t = 0.0;
     if (threadIdx.x == 0)
-        for (int k = 0; k < kTT / 32; ++k) t += red[k];
+        for (int k = 0; k < (int)(blockDim.x >> 5); ++k) t += red[k];
     return t;  // valid on thread 0
 }
 
@@ -75,108 +72,125 @@ __device__ __forceinline__ float rel_contrib(const TrainArgs& a, uint32_t i) {
     return r < a.loss_clamp ? r : a.loss_clamp;
 }
 
-using simt::kLd;
+using simt::at;
 using simt::kTM;
 
 // activation tile rows and weight-chunk floats of the training kernels
 template <int W>
 struct TrShape {
+    static constexpr int kThr = simt::threads_of(W);
     static constexpr int kRows = simt::imax(stat_in_of(W), W);
-    static constexpr int kChunk = simt::kKC * simt::imax(stat_in_of(W), W);
-    static constexpr size_t kSmem = sizeof(float) * ((size_t)kRows * kLd + 2 * kChunk);
+    static constexpr int kChunk = simt::kKC * W;
+    static constexpr size_t kSmem = sizeof(float) * ((size_t)kRows * kTM + 2 * kChunk);
 };
 
 // forward layer: ReLU (LeakyReLU for the reference network, W = 32) in place, and the activations
-// to scratch rows row0 + n (samples i0 ..)
+// to scratch rows row0 + n (samples i0 ..). Bit 8 j + i of `pos` tells whether the thread's j-th
+// neuron is positive for its i-th sample: the backward layers give a thread the same neurons and
+// samples, so their masks come from these registers.
 template <int W>
-__device__ __forceinline__ void fwd_layer(const float* __restrict__ wt, int k_rows, int k_eff,
-                                          float* tile, float* wch, int tid, float* scr,
-                                          uint32_t ld, uint32_t i0, uint32_t row0, bool store) {
-    simt::tile_gemm<W>(wt, k_rows, k_eff, tile, wch, tid, [&](int n, int m0, const float* v) {
-        float r[8];
+__device__ __forceinline__ void fwd_layer(const float* __restrict__ wt, int k_eff, float* tile,
+                                          float* wch, int tid, float* scr, uint32_t ld, uint32_t i0,
+                                          uint32_t row0, bool store, unsigned long long& pos) {
+    unsigned long long bits = 0;
+    simt::tile_gemm<W, TrShape<W>::kThr>(
+        wt, W, k_eff, tile, wch, tid, [&](int j, int n, int m0, const float* v) {
+            float r[8];
+            uint32_t b = 0;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) r[i] = W == 32 ? leaky(v[i]) : fmaxf(v[i], 0.f);
-        simt::tile_store8(tile, n, m0, r);
-        if (store) {
-            float* g = scr + (size_t)(row0 + n) * ld + i0 + m0;
+            for (int i = 0; i < 8; ++i) {
+                r[i] = W == 32 ? leaky(v[i]) : fmaxf(v[i], 0.f);
+                b |= (v[i] > 0.f ? 1u : 0u) << i;
+            }
+            bits |= (unsigned long long)b << (8 * j);
+            simt::tile_store8(tile, n, m0, r);
+            if (store) {
+                float* g = scr + (size_t)(row0 + n) * ld + i0 + m0;
+                *reinterpret_cast<float4*>(g) = make_float4(r[0], r[1], r[2], r[3]);
+                *reinterpret_cast<float4*>(g + 4) = make_float4(r[4], r[5], r[6], r[7]);
+            }
+        });
+    pos = bits;
+}
+
+// backward layer through row-major W [outputs of the forward layer][W = its inputs]:
+// delta_in[n][m] = (sum_k W[k][n] delta_out[k][m]) times the activation's slope (ReLU: 1 or 0;
+// LeakyReLU: 1 or 0.01) by the forward layer's `pos` bits; in place, and to scratch rows out0 + n
+template <int W>
+__device__ __forceinline__ void bwd_layer(const float* __restrict__ w, float* tile, float* wch,
+                                          int tid, float* scr, uint32_t ld, uint32_t i0,
+                                          uint32_t out0, unsigned long long pos) {
+    simt::tile_gemm<W, TrShape<W>::kThr>(
+        w, W, W, tile, wch, tid, [&](int j, int n, int m0, const float* v) {
+            float r[8];
+            const uint32_t b = (uint32_t)(pos >> (8 * j));
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                r[i] = (b >> i) & 1u ? v[i] : (W == 32 ? 0.01f * v[i] : 0.f);
+            simt::tile_store8(tile, n, m0, r);
+            float* g = scr + (size_t)(out0 + n) * ld + i0 + m0;
             *reinterpret_cast<float4*>(g) = make_float4(r[0], r[1], r[2], r[3]);
             *reinterpret_cast<float4*>(g + 4) = make_float4(r[4], r[5], r[6], r[7]);
-        }
-    });
+        });
 }
 
-// backward layer through row-major W [k_rows = outputs of the forward layer][W = its inputs]:
-// delta_in[n][m] = (sum_k W[k][n] delta_out[k][m]) times the activation's slope at the forward
-// activation stored in scratch rows mask0 + n (ReLU: 1 or 0; LeakyReLU: 1 or 0.01); in place, and
-// to scratch rows out0 + n
-template <int W>
-__device__ __forceinline__ void bwd_layer(const float* __restrict__ w, int k_rows, float* tile,
-                                          float* wch, int tid, float* scr, uint32_t ld, uint32_t i0,
-                                          uint32_t mask0, uint32_t out0) {
-    simt::tile_gemm<W>(w, k_rows, k_rows, tile, wch, tid, [&](int n, int m0, const float* v) {
-        const float* h = scr + (size_t)(mask0 + n) * ld + i0 + m0;
-        const float4 h0 = *reinterpret_cast<const float4*>(h);
-        const float4 h1 = *reinterpret_cast<const float4*>(h + 4);
-        const float hv[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
-        float r[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) r[i] = hv[i] > 0.f ? v[i] : (W == 32 ? 0.01f * v[i] : 0.f);
-        simt::tile_store8(tile, n, m0, r);
-        float* g = scr + (size_t)(out0 + n) * ld + i0 + m0;
-        *reinterpret_cast<float4*>(g) = make_float4(r[0], r[1], r[2], r[3]);
-        *reinterpret_cast<float4*>(g + 4) = make_float4(r[4], r[5], r[6], r[7]);
-    });
-}
-
-// y[o] = sum_k wt[k][o] tile[k][m] for a narrow output layer (wt [W][4])
+// The delta of the last hidden layer in column m of the tile (which holds that layer's
+// activations): d[k] = sum_o w[o][k] g[o] times the activation's slope; w is the row-major output
+// layer [OUT][W]. Also to scratch rows at dl (stride ld) when store is set.
 template <int W, int OUT>
-__device__ __forceinline__ void narrow_out(const float* __restrict__ wt, const float* tile, int m,
-                                           float* y) {
-    constexpr int OP = (OUT + 3) / 4 * 4;   // wt is [W][OUT rounded up to 4]
-    float acc[OUT];
+__device__ __forceinline__ void last_delta(const float* __restrict__ w, const float* g, float* tile,
+                                           int m, float* dl, uint32_t ld, bool store) {
+    constexpr bool REF = W == 32;
+#pragma unroll 2
+    for (int k = 0; k < W; k += 4) {
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int o = 0; o < OUT; ++o) acc[o] = 0.f;
-#pragma unroll 4
-    for (int k = 0; k < W; ++k) {
-        const float x = tile[k * kLd + m];
+        for (int o = 0; o < OUT; ++o) {
+            const float4 wv = __ldg(reinterpret_cast<const float4*>(w + o * W + k));
+            acc[0] = fmaf(wv.x, g[o], acc[0]);
+            acc[1] = fmaf(wv.y, g[o], acc[1]);
+            acc[2] = fmaf(wv.z, g[o], acc[2]);
+            acc[3] = fmaf(wv.w, g[o], acc[3]);
+        }
 #pragma unroll
-        for (int q = 0; q < OP / 4; ++q) {
-            const float4 w = __ldg(reinterpret_cast<const float4*>(wt + OP * k + 4 * q));
-            const float wv[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-                if (4 * q + e < OUT) acc[4 * q + e] = fmaf(wv[e], x, acc[4 * q + e]);
+        for (int e = 0; e < 4; ++e) {
+            float& x = tile[at(k + e, m)];
+            const float d = x > 0.f ? acc[e] : (REF ? 0.01f * acc[e] : 0.f);
+            x = d;
+            if (store) dl[(size_t)(k + e) * ld] = d;
         }
     }
-#pragma unroll
-    for (int o = 0; o < OUT; ++o) y[o] = acc[o];
 }
 
-// The StatNet step and the RRSNet forward sums on 64-sample tiles (128 threads): encoding (two
-// threads per sample), the forward layers as tile GEMMs storing every activation, the loss
-// gradient, the backward layers as tile GEMMs through the row-major weights (masks from the
-// stored activations), the input gradient of the 32 hash lanes, the hash-grid scatter (two
-// threads per sample, eight levels each), then the glue and the RRSNet forward for the sums.
+// The StatNet step and the RRSNet forward sums on 64-sample tiles: encoding, the forward layers as
+// tile GEMMs storing every activation, the loss gradient, the backward layers as tile GEMMs
+// through the row-major weights, the input gradient of the hash lanes, the hash-grid scatter, then
+// the glue and the RRSNet forward for the sums. Per-sample phases run one thread per sample (64
+// threads per CTA); the 128-wide networks' CTAs have 128 threads and split encoding and scatter
+// over two per sample.
+// 64 x 2, 262,144 samples: 315 us beside 89 us of encoding and 185 us of scatter (kernels of their
+// own, the scatter overlapped), against 735 us for one kernel that did all three with 24 warps per
+// SM waiting for the gathers (330 us of it) and for the reductions (175 us).
 template <int WS, int HS, int WR, int HR>
-__global__ void __launch_bounds__(simt::kThr) k_train_stat(const __grid_constant__ TrainArgs a) {
+__global__ void __launch_bounds__(TrShape<WS>::kThr, WS == 128 ? 4 : 8)
+    k_train_stat(const __grid_constant__ TrainArgs a) {
     static_assert(WS == WR, "one tile shape for both networks");
     constexpr bool REF = WS == 32;             // the reference's shipped network
     constexpr int SIN = stat_in_of(WS), SOUT = stat_out_of(WS);
-    constexpr int NLH = REF ? kRefLevels / 2 : 8;   // hash levels per thread (two per sample)
     constexpr int X1 = REF ? kRefRrsLanes : 10;     // live RRSNet input lanes
     using S = TrShape<WS>;
+    constexpr int TPS = S::kThr / kTM;              // threads per sample
     extern __shared__ float4 smem4[];
     float* tile = reinterpret_cast<float*>(smem4);
-    float* wch = tile + S::kRows * kLd;
-    __shared__ double red[kTT / 32];
+    float* wch = tile + S::kRows * kTM;
+    __shared__ double red[S::kThr / 32];
     const int tid = threadIdx.x;
     const int m = tid & (kTM - 1);
     const bool lead = tid < kTM;
-    const int half = tid >> 6;
+    const bool lo = TPS == 1 || lead, hi = TPS == 1 || !lead;   // this thread's share of the lanes
     const uint32_t ld = a.ld;
     float* scr = a.act;
     double lossS = 0.0, sumV = 0.0, sumC = 0.0, sumR = 0.0;
-    const float2* table = reinterpret_cast<const float2*>(a.table);
     // forward (transposed) and backward (row-major) layer images
     const float* ts = a.wt_stat;
     const float* ts_out = ts + (size_t)SIN * WS + (size_t)(HS - 1) * WS * WS;
@@ -190,64 +204,51 @@ __global__ void __launch_bounds__(simt::kThr) k_train_stat(const __grid_constant
         const uint32_t i0 = u * kTM, i = i0 + m;
         const bool valid = i < a.n;
         __syncthreads();   // the previous tile's column reads are over
-        // ---- encode: lanes 0..55 of this sample's column (half 0: levels 0-7 + SH, 1: 8-15 +
-        //      misc), copied to the x0 scratch rows ----
-        float p[3] = {0.f, 0.f, 0.f};
+        // ---- the input tile: hash lanes from the encoding kernel's x0 rows, the other lanes here
+        //      (and to their x0 rows) ----
+        constexpr int LANES = REF ? 32 : 56, HL = REF ? 16 : 32;
+        simt::load_rows<HL, S::kThr>(scr + (size_t)a.r_x0 * ld + i0, ld, tile, tid);
+        simt::cp_async_commit();
         if (valid) {
-            norm_pos(a.enc, a.v.pos, i, p);
-#pragma unroll 2
-            for (int l = half * NLH; l < half * NLH + NLH; ++l) {
-                const LevelDev L = a.enc.lv[l];
-                const CellCoord c = cell_of(p, L.res);
-                float f0 = 0.f, f1 = 0.f;
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    const uint32_t row = grid_row(L, a.enc.hash_mask, c.ix + (k & 1),
-                                                  c.iy + ((k >> 1) & 1), c.iz + ((k >> 2) & 1));
-                    const float2 tv = __ldg(table + row);
-                    const float w = corner_weight(c, k);
-                    f0 += w * tv.x;
-                    f1 += w * tv.y;
-                }
-                tile[(2 * l) * kLd + m] = f0;
-                tile[(2 * l + 1) * kLd + m] = f1;
-            }
+            float* x0 = scr + (size_t)(a.r_x0 + HL) * ld + i;
+            auto put = [&](int k, float x) {
+                tile[at(HL + k, m)] = x;
+                x0[(size_t)k * ld] = x;
+            };
             if (REF) {
-                // the reference network: direction blobs (half 0) or roughness blob (half 1)
+                // the reference network: direction blobs (lo) and roughness blob (hi)
                 float blob[16];
                 ref_blob_lanes(a.v, i, blob);
 #pragma unroll
-                for (int k = 0; k < 8; ++k)
-                    tile[(16 + 8 * half + k) * kLd + m] = half ? blob[8 + k] : blob[k];
-            } else if (half == 0) {
-                float sh[16];
-                const size_t i3 = 3 * (size_t)i;
-                sh16(a.v.wi[i3], a.v.wi[i3 + 1], a.v.wi[i3 + 2], sh);
-#pragma unroll
-                for (int k = 0; k < 16; ++k) tile[(32 + k) * kLd + m] = sh[k];
+                for (int k = 0; k < 16; ++k)
+                    if (k < 8 ? lo : hi) put(k, blob[k]);
             } else {
-                float mm[16];
-                misc_lanes(a.v, i, mm);
+                if (lo) {
+                    float sh[16];
+                    const size_t i3 = 3 * (size_t)i;
+                    sh16(a.v.wi[i3], a.v.wi[i3 + 1], a.v.wi[i3 + 2], sh);
 #pragma unroll
-                for (int k = 0; k < 8; ++k) tile[(48 + k) * kLd + m] = mm[k];
+                    for (int k = 0; k < 16; ++k) put(k, sh[k]);
+                }
+                if (hi) {
+                    float mm[16];
+                    misc_lanes(a.v, i, mm);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) put(16 + k, mm[k]);
+                }
             }
-            const int hl = 2 * NLH;                              // hash lanes of this half
-            for (int k = half * hl; k < half * hl + hl; ++k)
-                scr[(size_t)(a.r_x0 + k) * ld + i] = tile[k * kLd + m];
-            const int q0 = REF ? 16 + 8 * half : (half ? 48 : 32);
-            const int q1 = REF ? q0 + 8 : (half ? 56 : 48);      // the other lanes of this half
-            for (int k = q0; k < q1; ++k) scr[(size_t)(a.r_x0 + k) * ld + i] = tile[k * kLd + m];
         } else {
-            constexpr int LANES = REF ? 32 : 56;
-            for (int k = half * LANES / 2; k < (half + 1) * LANES / 2; ++k) tile[k * kLd + m] = 0.f;
+            constexpr int NO = LANES - HL;       // non-hash lanes; `hi` owns the last 8
+            for (int k = lo ? 0 : NO - 8; k < (hi ? NO : NO - 8); ++k) tile[at(HL + k, m)] = 0.f;
         }
 
         // ---- StatNet forward, every hidden activation to scratch ----
-        fwd_layer<WS>(ts, SIN, REF ? 32 : 56, tile, wch, tid, scr, ld, i0, a.r_hs, true);
-#pragma unroll 1
+        unsigned long long pos[HS];
+        fwd_layer<WS>(ts, LANES, tile, wch, tid, scr, ld, i0, a.r_hs, true, pos[0]);
+#pragma unroll
         for (int h = 1; h < HS; ++h)
-            fwd_layer<WS>(ts + (size_t)SIN * WS + (size_t)(h - 1) * WS * WS, WS, WS, tile, wch,
-                          tid, scr, ld, i0, a.r_hs + h * WS, true);
+            fwd_layer<WS>(ts + (size_t)SIN * WS + (size_t)(h - 1) * WS * WS, WS, tile, wch, tid,
+                          scr, ld, i0, a.r_hs + h * WS, true, pos[h]);
 
         // ---- output, loss gradient, and the delta of the last hidden layer (own column) ----
         float y[SOUT];
@@ -255,7 +256,7 @@ __global__ void __launch_bounds__(simt::kThr) k_train_stat(const __grid_constant
         for (int k = 0; k < SOUT; ++k) y[k] = 0.f;
         SampleMul mu{1.f, 1.f, 1.f, 0.f};
         if (lead) {
-            narrow_out<WS, SOUT>(ts_out, tile, m, y);
+            simt::narrow_out<WS, SOUT>(ts_out, tile, m, y);
             float g[SOUT];
 #pragma unroll
             for (int k = 0; k < SOUT; ++k) g[k] = 0.f;
@@ -289,42 +290,23 @@ __global__ void __launch_bounds__(simt::kThr) k_train_stat(const __grid_constant
                     }
                 }
             }
-            // d h_last = W_out^T g times the activation's slope at h_last (this column)
-            float* dl = scr + (size_t)(a.r_dhs + (HS - 1) * WS) * ld + i;
-#pragma unroll 4
-            for (int k = 0; k < WS; ++k) {
-                float acc = 0.f;
-#pragma unroll
-                for (int o = 0; o < SOUT; ++o) acc = fmaf(rs_out[o * WS + k], g[o], acc);
-                const float dk = tile[k * kLd + m] > 0.f ? acc : (REF ? 0.01f * acc : 0.f);
-                tile[k * kLd + m] = dk;
-                if (valid) dl[(size_t)k * ld] = dk;
-            }
+            last_delta<WS, SOUT>(rs_out, g, tile, m,
+                                 scr + (size_t)(a.r_dhs + (HS - 1) * WS) * ld + i, ld, valid);
         }
 
         // ---- backward through the hidden layers, then the hash-lane gradients ----
-#pragma unroll 1
+#pragma unroll
         for (int h = HS - 1; h >= 1; --h)
-            bwd_layer<WS>(rs + (size_t)SIN * WS + (size_t)(h - 1) * WS * WS, WS, tile, wch,
-                          tid, scr, ld, i0, a.r_hs + (h - 1) * WS, a.r_dhs + (h - 1) * WS);
-        simt::tile_gemm<SIN>(rs, WS, WS, tile, wch, tid, [&](int n, int m0, const float* v) {
-            simt::tile_store8(tile, n, m0, v);
+            bwd_layer<WS>(rs + (size_t)SIN * WS + (size_t)(h - 1) * WS * WS, tile, wch, tid, scr,
+                          ld, i0, a.r_dhs + (h - 1) * WS, pos[h - 1]);
+        // straight to scratch: the level-major scatter applies them
+        simt::tile_gemm<32, S::kThr>(rs, SIN, WS, tile, wch, tid,
+                                     [&](int, int n, int m0, const float* v) {
+            if (n >= HL) return;
+            float* g = scr + (size_t)(a.r_dx + n) * ld + i0 + m0;
+            *reinterpret_cast<float4*>(g) = make_float4(v[0], v[1], v[2], v[3]);
+            *reinterpret_cast<float4*>(g + 4) = make_float4(v[4], v[5], v[6], v[7]);
         });
-
-        // ---- hash-grid scatter: two threads per sample, half the levels each ----
-        {
-            const unsigned lanes = valid_lanes(i0 + (uint32_t)(m & ~31), a.n);
-            if (valid) {
-#pragma unroll 2
-                for (int l = half * NLH; l < half * NLH + NLH; ++l) {
-                    const LevelDev L = a.enc.lv[l];
-                    const CellCoord c = cell_of(p, L.res);
-                    warp_scatter_level(a.table_grad, L, a.enc.hash_mask, c, tile[(2 * l) * kLd + m],
-                                       tile[(2 * l + 1) * kLd + m], lanes);
-                }
-            }
-        }
-        __syncthreads();
 
         // ---- glue and the RRSNet forward for the batch sums ----
         if (a.train_rrs) {
@@ -334,18 +316,19 @@ __global__ void __launch_bounds__(simt::kThr) k_train_stat(const __grid_constant
                 else glue16(a.fp, y, a.v, valid ? i : 0u, x1);
 #pragma unroll
                 for (int k = 0; k < X1; ++k) {
-                    tile[k * kLd + m] = valid ? x1[k] : 0.f;
+                    tile[at(k, m)] = valid ? x1[k] : 0.f;
                     if (valid) scr[(size_t)(a.r_x1 + k) * ld + i] = x1[k];
                 }
             }
-            fwd_layer<WR>(tr, kRrsIn, X1, tile, wch, tid, scr, ld, i0, 0, false);
+            unsigned long long unused;
+            fwd_layer<WR>(tr, X1, tile, wch, tid, scr, ld, i0, 0, false, unused);
 #pragma unroll 1
             for (int h = 1; h < HR; ++h)
-                fwd_layer<WR>(tr + (size_t)kRrsIn * WR + (size_t)(h - 1) * WR * WR, WR, WR, tile,
-                              wch, tid, scr, ld, i0, 0, false);
+                fwd_layer<WR>(tr + (size_t)kRrsIn * WR + (size_t)(h - 1) * WR * WR, WR, tile, wch,
+                              tid, scr, ld, i0, 0, false, unused);
             if (lead && valid) {
                 float raw;
-                narrow_out<WR, 1>(tr_out, tile, m, &raw);
+                simt::narrow_out<WR, 1>(tr_out, tile, m, &raw);
                 const float q = act_sigma(raw);
                 const float r = rel_contrib(a, i);
                 if (a.lw.active) {
@@ -375,23 +358,33 @@ __global__ void __launch_bounds__(simt::kThr) k_train_stat(const __grid_constant
 // The RRSNet step on 64-sample tiles: the forward layers again (activations to scratch), the
 // loss gradient with the batch's V and C, and the backward layers.
 template <int WR, int HR>
-__global__ void __launch_bounds__(simt::kThr) k_train_rrs(const __grid_constant__ TrainArgs a) {
+__global__ void __launch_bounds__(TrShape<WR>::kThr, WR == 128 ? 4 : 8)
+    k_train_rrs(const __grid_constant__ TrainArgs a) {
     constexpr bool REF = WR == 32;             // the reference's shipped network
     constexpr int X1 = REF ? kRefRrsLanes : 10;
     using S = TrShape<WR>;
     extern __shared__ float4 smem4[];
     float* tile = reinterpret_cast<float*>(smem4);
-    float* wch = tile + S::kRows * kLd;
-    __shared__ double s_tot[4];
+    float* wch = tile + S::kRows * kTM;
+    __shared__ double s_tot[4], s_red[4][S::kThr / 4];
     const int tid = threadIdx.x;
     const int m = tid & (kTM - 1);
     const bool lead = tid < kTM;
     const uint32_t ld = a.ld;
     float* scr = a.act;
-    if (tid < 4) {
+    // the batch sums of the StatNet kernel's CTA partials, in the same order in every CTA: slices of
+    // rows b = tid / 4 (mod threads / 4), then the slices (one serial sum per column took 40 us)
+    {
         double t = 0.0;
-        for (uint32_t b = 0; b < a.part_n; ++b) t += a.part[4 * b + tid];
-        s_tot[tid] = t;
+#pragma unroll 8
+        for (uint32_t b = tid >> 2; b < a.part_n; b += S::kThr / 4) t += a.part[4 * b + (tid & 3)];
+        s_red[tid & 3][tid >> 2] = t;
+        __syncthreads();
+        if (tid < 4) {
+            t = 0.0;
+            for (int k = 0; k < S::kThr / 4; ++k) t += s_red[tid][k];
+            s_tot[tid] = t;
+        }
     }
     __syncthreads();
     const double Vm = s_tot[1] / (double)a.n, Cm = s_tot[2] / (double)a.n;
@@ -415,18 +408,19 @@ __global__ void __launch_bounds__(simt::kThr) k_train_rrs(const __grid_constant_
         if (lead) {
 #pragma unroll
             for (int k = 0; k < X1; ++k)
-                tile[k * kLd + m] = valid ? scr[(size_t)(a.r_x1 + k) * ld + i] : 0.f;
+                tile[at(k, m)] = valid ? scr[(size_t)(a.r_x1 + k) * ld + i] : 0.f;
         }
-        fwd_layer<WR>(tr, kRrsIn, X1, tile, wch, tid, scr, ld, i0, a.r_hr, true);
-#pragma unroll 1
+        unsigned long long pos[HR];
+        fwd_layer<WR>(tr, X1, tile, wch, tid, scr, ld, i0, a.r_hr, true, pos[0]);
+#pragma unroll
         for (int h = 1; h < HR; ++h)
-            fwd_layer<WR>(tr + (size_t)kRrsIn * WR + (size_t)(h - 1) * WR * WR, WR, WR, tile, wch,
-                          tid, scr, ld, i0, a.r_hr + h * WR, true);
+            fwd_layer<WR>(tr + (size_t)kRrsIn * WR + (size_t)(h - 1) * WR * WR, WR, tile, wch, tid,
+                          scr, ld, i0, a.r_hr + h * WR, true, pos[h]);
         if (lead) {
             float draw = 0.f;
             if (valid) {
                 float raw;
-                narrow_out<WR, 1>(tr_out, tile, m, &raw);
+                simt::narrow_out<WR, 1>(tr_out, tile, m, &raw);
                 const float q = act_sigma(raw);
                 const float r = rel_contrib(a, i);
                 float dq;
@@ -440,20 +434,13 @@ __global__ void __launch_bounds__(simt::kThr) k_train_rrs(const __grid_constant_
                 draw = dq * act_sigma_grad(raw);
                 scr[(size_t)a.r_draw * ld + i] = draw;
             }
-            // d g_last = V_out^T draw, masked by g_last (this column of the tile)
-            float* dl = scr + (size_t)(a.r_dhr + (HR - 1) * WR) * ld + i;
-#pragma unroll 4
-            for (int k = 0; k < WR; ++k) {
-                const float dk = tile[k * kLd + m] > 0.f ? rr_out[k] * draw
-                                                         : (REF ? 0.01f * (rr_out[k] * draw) : 0.f);
-                tile[k * kLd + m] = dk;
-                if (valid) dl[(size_t)k * ld] = dk;
-            }
+            last_delta<WR, 1>(rr_out, &draw, tile, m,
+                              scr + (size_t)(a.r_dhr + (HR - 1) * WR) * ld + i, ld, valid);
         }
-#pragma unroll 1
+#pragma unroll
         for (int h = HR - 1; h >= 1; --h)
-            bwd_layer<WR>(rr + (size_t)kRrsIn * WR + (size_t)(h - 1) * WR * WR, WR, tile, wch, tid,
-                          scr, ld, i0, a.r_hr + (h - 1) * WR, a.r_dhr + (h - 1) * WR);
+            bwd_layer<WR>(rr + (size_t)kRrsIn * WR + (size_t)(h - 1) * WR * WR, tile, wch, tid, scr,
+                          ld, i0, a.r_dhr + (h - 1) * WR, pos[h - 1]);
     }
 }
 
@@ -536,13 +523,6 @@ constexpr int kWPitch = kWS + 4;
 constexpr int kWRows = 128;      // largest tile: 64 delta + 64 activation rows
 constexpr size_t kWSmem = sizeof(float) * (size_t)kWStages * kWRows * kWPitch;
 
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b,
-                                                   unsigned long long c) {
-    unsigned long long d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-
 // The whole (job, chunk): rows arrive as 16-byte cp.async copies (samples past the chunk's end
 // zero-filled), three stages deep; a thread reads 4 samples of its RU delta and 4 activation rows
 // as 16-byte words and adds the products of the even and odd samples as FP32 pairs (two FMAs per
@@ -610,7 +590,7 @@ __device__ __forceinline__ void wgrad_tile(const WGradArgs& a, const WJob& j, fl
                     *reinterpret_cast<const ulonglong2*>(D + u * TY * kWPitch + 4 * q);
 #pragma unroll
                 for (int w = 0; w < 4; ++w)
-                    acc[u][w] = fma2(d.y, x[w].y, fma2(d.x, x[w].x, acc[u][w]));
+                    acc[u][w] = simt::fma2(d.y, x[w].y, simt::fma2(d.x, x[w].x, acc[u][w]));
             }
         }
     }
@@ -622,7 +602,7 @@ __device__ __forceinline__ void wgrad_tile(const WGradArgs& a, const WJob& j, fl
 #pragma unroll
         for (int w = 0; w < 4; ++w) {
             float e, o;
-            asm("mov.b64 {%0, %1}, %2;" : "=f"(e), "=f"(o) : "l"(acc[u][w]));
+            simt::unpack2f(acc[u][w], e, o);
             sm[grp * TM * TN + (ty + u * TY) * TN + tx + w * TX] = e + o;
         }
     __syncthreads();
@@ -824,8 +804,11 @@ __global__ void k_ema(const __grid_constant__ EmaArgs a) {
     }
 }
 
-template <int WS, int HS, int WR, int HR>
-cudaError_t launch_train(nrrs_ctx* ctx, TrainArgs& a, cudaStream_t s) {
+// after_stat() is called once the StatNet kernel is launched (the step forks the table-gradient
+// scatter there)
+template <int WS, int HS, int WR, int HR, class AfterStat>
+cudaError_t launch_train(nrrs_ctx* ctx, TrainArgs& a, cudaStream_t s, AfterStat after_stat) {
+    constexpr int kThr = TrShape<WS>::kThr;
     const size_t smem = TrShape<WS>::kSmem;
     auto ks = k_train_stat<WS, HS, WR, HR>;
     auto kr = k_train_rrs<WR, HR>;
@@ -834,23 +817,24 @@ cudaError_t launch_train(nrrs_ctx* ctx, TrainArgs& a, cudaStream_t s) {
         e = cudaFuncSetAttribute(kr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const uint32_t tiles = (a.n + kTM - 1) / kTM;
-    uint32_t grid = (uint32_t)(ctx->sm_count * resident_ctas((const void*)ks, simt::kThr, smem, 16));
+    uint32_t grid = (uint32_t)(ctx->sm_count * resident_ctas((const void*)ks, kThr, smem, 16));
     if (grid > tiles) grid = tiles;
     a.part_n = grid;
     {
         ProfScope ps(ctx, NRRS_KERNEL_TRAIN_STAT, s);
-        ks<<<grid, simt::kThr, smem, s>>>(a);
+        ks<<<grid, kThr, smem, s>>>(a);
     }
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if ((e = after_stat()) != cudaSuccess) return e;
     {
         ProfScope ps(ctx, NRRS_KERNEL_TRAIN_RRS, s);
-        kr<<<grid, simt::kThr, smem, s>>>(a);
+        kr<<<grid, kThr, smem, s>>>(a);
     }
     return cudaGetLastError();
 }
 
 struct Layout {
-    uint32_t r_x0, r_hs, r_dhs, r_dy, r_x1, r_hr, r_dhr, r_draw, rows;
+    uint32_t r_x0, r_hs, r_dhs, r_dx, r_dy, r_x1, r_hr, r_dhr, r_draw, rows;
 };
 
 Layout layout_of(const nrrs_config& c) {
@@ -860,6 +844,7 @@ Layout layout_of(const nrrs_config& c) {
     L.r_x0 = r; r += ref ? kRefStatIn : 56;
     L.r_hs = r; r += c.statnet_hidden * c.statnet_width;
     L.r_dhs = r; r += c.statnet_hidden * c.statnet_width;
+    L.r_dx = r; r += 2 * c.n_levels;
     L.r_dy = r; r += ref ? 8 : 4;
     L.r_x1 = r; r += 16;
     L.r_hr = r; r += c.rrsnet_hidden * c.rrsnet_width;
@@ -971,8 +956,11 @@ int train_step_impl(nrrs_ctx* ctx, const VertexPtrs& v, const float* target, uin
     const bool train_rrs = c.step >= 3;
     cudaError_t e;
 
-    // gradients of this step only
-    e = cudaMemsetAsync(ctx->grads, 0, sizeof(float) * ctx->n_params, s);
+    // gradients of this step only: the scatter zeroes the table's, the weight gradients write
+    // theirs, and an untrained RRSNet's are zero
+    e = train_rrs ? cudaSuccess
+                  : cudaMemsetAsync(ctx->grads + ctx->n_table + ctx->n_stat, 0,
+                                    sizeof(float) * ctx->n_rrs, s);
     if (e != cudaSuccess) {
         ctx->last_error = std::string("train memset: ") + cudaGetErrorString(e);
         return NRRS_ERR_CUDA;
@@ -983,34 +971,71 @@ int train_step_impl(nrrs_ctx* ctx, const VertexPtrs& v, const float* target, uin
     a.target = target;
     a.n = n;
     a.ld = ld;
-    a.enc = ctx->enc;
     a.fp.stat_eps = c.stat_eps;
     a.fp.ref_eps = c.ref_eps;
     a.loss_clamp = c.loss_clamp_max;
     a.cost_offset = c.cost_offset;
     a.train_rrs = train_rrs;
-    a.table = ctx->params;
-    a.table_grad = ctx->grads;
     a.wt_stat = ctx->wt;
     a.wt_rrs = ctx->wt + ctx->wt_rrs_offset;
     a.w_stat = ctx->wrow;
     a.w_rrs = ctx->wrow + ctx->n_stat;
     a.act = act;
-    a.r_x0 = L.r_x0; a.r_hs = L.r_hs; a.r_dhs = L.r_dhs; a.r_dy = L.r_dy;
+    a.r_x0 = L.r_x0; a.r_hs = L.r_hs; a.r_dhs = L.r_dhs; a.r_dx = L.r_dx; a.r_dy = L.r_dy;
     a.r_x1 = L.r_x1; a.r_hr = L.r_hr; a.r_dhr = L.r_dhr; a.r_draw = L.r_draw;
     a.part = part;
     a.loss_out = loss_dev ? loss_dev : ctx->loss_dev;
     if (lw) a.lw = *lw;
 
-    if (c.statnet_width == 64 && c.statnet_hidden == 2)
-        e = launch_train<64, 2, 64, 2>(ctx, a, s);
-    else if (c.statnet_width == 64 && c.statnet_hidden == 3)
-        e = launch_train<64, 3, 64, 3>(ctx, a, s);
-    else if (c.statnet_width == 32)   // the reference network
-        e = launch_train<32, 3, 32, 3>(ctx, a, s);
-    else
-        e = launch_train<128, 3, 128, 3>(ctx, a, s);
+    // the hash rows of x0, level-major
+    EncodeF32Args ea{};
+    ea.enc = ctx->enc;
+    ea.segs.n = 1;
+    ea.segs.s[0].count = n;
+    ea.segs.total_tiles = (n + kTile - 1) / kTile;
+    ea.pos = v.pos;
+    ea.table = ctx->params;
+    ea.out = act + (size_t)L.r_x0 * ld;
+    ea.tile_stride = kTile;
+    ea.lane_stride = ld;
+    ea.tile_end = ea.segs.total_tiles;
+    {
+        ProfScope ps(ctx, NRRS_KERNEL_TRAIN_ENCODE, s);
+        e = launch_encode_f32(ea, ctx->sm_count, s);
+    }
     if (e != cudaSuccess) {
+        ctx->last_error = std::string("training encoding launch: ") + cudaGetErrorString(e);
+        return NRRS_ERR_CUDA;
+    }
+    // The scatter is bound by L2 reductions, the RRSNet kernel and the weight gradients by the
+    // FP32 pipe: it runs beside them on the context's side stream, forked after the StatNet
+    // kernel and joined before Adam (nothing in between reads the table gradient).
+    bool forked = false;
+    auto after_stat = [&]() -> cudaError_t {
+        cudaError_t ef = cudaEventRecord(ctx->ev_fork, s);
+        if (ef == cudaSuccess) ef = cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0);
+        if (ef != cudaSuccess) return ef;
+        forked = true;
+        ef = launch_scatter_table(ctx, v.pos, n,
+                                  LaneGrads{act + (size_t)L.r_dx * ld, 2 * (size_t)ld, 1, ld, 1.0f},
+                                  ctx->side);
+        const cudaError_t ej = cudaEventRecord(ctx->ev_join, ctx->side);
+        return ef != cudaSuccess ? ef : ej;
+    };
+    auto join = [&]() {
+        if (forked) cudaStreamWaitEvent(s, ctx->ev_join, 0);
+        forked = false;
+    };
+    if (c.statnet_width == 64 && c.statnet_hidden == 2)
+        e = launch_train<64, 2, 64, 2>(ctx, a, s, after_stat);
+    else if (c.statnet_width == 64 && c.statnet_hidden == 3)
+        e = launch_train<64, 3, 64, 3>(ctx, a, s, after_stat);
+    else if (c.statnet_width == 32)   // the reference network
+        e = launch_train<32, 3, 32, 3>(ctx, a, s, after_stat);
+    else
+        e = launch_train<128, 3, 128, 3>(ctx, a, s, after_stat);
+    if (e != cudaSuccess) {
+        join();
         ctx->last_error = std::string("train launch: ") + cudaGetErrorString(e);
         return NRRS_ERR_CUDA;
     }
@@ -1060,6 +1085,7 @@ int train_step_impl(nrrs_ctx* ctx, const VertexPtrs& v, const float* target, uin
         e = launch_wreduce(partial, (uint32_t)chunks, (uint32_t)mlp, off, ctx->grads + ctx->n_table,
                            1.0f, s);
     }
+    join();  // the table gradient is complete on s from here
     if (e != cudaSuccess) {
         ctx->last_error = std::string("wgrad launch: ") + cudaGetErrorString(e);
         return NRRS_ERR_CUDA;

@@ -392,17 +392,15 @@ constexpr uint64_t kScatterGroupBytes = 40ull << 20;
 struct ScatterLvArgs {
     EncodeParams enc;
     const float* pos;
-    const float* dxs;
+    LaneGrads g;
     float* table_grad;
     uint32_t n;
-    float inv_n;
     uint32_t level_begin, level_end;
 };
 
 __global__ void __launch_bounds__(128) k_scatter_levels(const __grid_constant__ ScatterLvArgs a) {
     const uint32_t tiles = (a.n + 127) / 128;
     const uint32_t items = (a.level_end - a.level_begin) * tiles;
-    const float2* d = reinterpret_cast<const float2*>(a.dxs);
     for (uint32_t w = blockIdx.x; w < items; w += gridDim.x) {
         const uint32_t lq = w / tiles, t = w - lq * tiles;
         const uint32_t l = a.level_begin + lq;
@@ -410,10 +408,11 @@ __global__ void __launch_bounds__(128) k_scatter_levels(const __grid_constant__ 
         if (i >= a.n) continue;
         float p[3];
         norm_pos(a.enc, a.pos, i, p);
-        const float2 g = d[(size_t)l * a.n + i];
+        const float* d = a.g.dxs + l * a.g.level_stride + i * a.g.sample_stride;
+        const float g0 = d[0], g1 = d[a.g.comp_stride];
         const LevelDev L = a.enc.lv[l];
         const CellCoord c = cell_of(p, L.res);
-        warp_scatter_level(a.table_grad, L, a.enc.hash_mask, c, g.x * a.inv_n, g.y * a.inv_n,
+        warp_scatter_level(a.table_grad, L, a.enc.hash_mask, c, g0 * a.g.scale, g1 * a.g.scale,
                            valid_lanes(i - (threadIdx.x & 31u), a.n));
     }
 }
@@ -866,6 +865,52 @@ size_t train_tc_scratch_bytes(const nrrs_config& c, uint32_t n, int sm_count) {
            sizeof(float) * 32ull * n + 1024;
 }
 
+cudaError_t launch_scatter_table(nrrs_ctx* ctx, const float* pos, uint32_t n, const LaneGrads& g,
+                                 cudaStream_t s) {
+    // Level groups of at most kScatterGroupBytes of FP32 gradient, each zeroed right before its
+    // scatter: the zeroing writes whole sectors into L2, so the reductions that follow hit
+    // there. Zeroed at the start of the step, the slices were evicted by the kernels in between,
+    // and every first reduction into a sector read its zeros back from HBM as a random 32-byte
+    // access.
+    ScatterLvArgs sa{};
+    sa.enc = ctx->enc;
+    sa.pos = pos;
+    sa.g = g;
+    sa.table_grad = ctx->grads;
+    sa.n = n;
+    const uint32_t tiles = (n + 127) / 128;
+    const uint32_t g_max =
+        (uint32_t)(ctx->sm_count * resident_ctas((const void*)k_scatter_levels, 128, 0, 16));
+    const int nl = ctx->cfg.n_levels;
+    auto level_rows = [&](int l) -> uint64_t {
+        const LevelDev& lv = ctx->enc.lv[l];
+        const uint64_t r = (uint64_t)lv.res + 1;
+        return lv.dense ? r * r * r : (uint64_t)ctx->enc.hash_mask + 1;
+    };
+    cudaError_t e = cudaSuccess;
+    for (int l0 = 0; l0 < nl && e == cudaSuccess;) {
+        const uint64_t row0 = ctx->enc.lv[l0].offset;
+        uint64_t row1 = row0 + level_rows(l0);
+        int l1 = l0 + 1;
+        while (l1 < nl &&
+               (ctx->enc.lv[l1].offset + level_rows(l1) - row0) * 8u <= kScatterGroupBytes) {
+            row1 = ctx->enc.lv[l1].offset + level_rows(l1);
+            ++l1;
+        }
+        e = cudaMemsetAsync(ctx->grads + 2 * row0, 0, sizeof(float) * 2 * (row1 - row0), s);
+        if (e != cudaSuccess) break;
+        sa.level_begin = (uint32_t)l0;
+        sa.level_end = (uint32_t)l1;
+        const uint32_t items = (uint32_t)(l1 - l0) * tiles;
+        const uint32_t g_n = g_max < items ? g_max : items;
+        ProfScope ps(ctx, NRRS_KERNEL_TRAIN_SCATTER, s);
+        if (g_n) k_scatter_levels<<<g_n, 128, 0, s>>>(sa);
+        e = cudaGetLastError();
+        l0 = l1;
+    }
+    return e;
+}
+
 cudaError_t launch_wreduce(const float* partial, uint32_t chunks, uint32_t stride, uint32_t count,
                            float* grad, float scale, cudaStream_t s);
 int train_step_tc(nrrs_ctx* ctx, const VertexPtrs& v, const float* target, uint32_t n,
@@ -964,50 +1009,9 @@ int train_step_tc(nrrs_ctx* ctx, const VertexPtrs& v, const float* target, uint3
     // and nothing before Adam reads the table gradient, so it runs on the context's side
     // stream, forked after the StatNet launch, while the RRSNet kernels and the weight
     // gradients run here; the step joins it before Adam (or before returning the gradients).
-    // Level groups of at most kScatterGroupBytes of FP32 gradient, each zeroed right before its
-    // scatter: the zeroing writes whole sectors into L2, so the reductions that follow hit
-    // there. Zeroed at the start of the step, the slices were evicted by the kernels in between,
-    // and every first reduction into a sector read its zeros back from HBM as a random 32-byte
-    // access.
     auto scatter_table = [&](cudaStream_t ss) -> cudaError_t {
-        ScatterLvArgs sa{};
-        sa.enc = ctx->enc;
-        sa.pos = v.pos;
-        sa.dxs = dxs;
-        sa.table_grad = ctx->grads;
-        sa.n = n;
-        sa.inv_n = a.inv_n;
-        const uint32_t tiles = (n + 127) / 128;
-        const uint32_t g_max =
-            (uint32_t)(ctx->sm_count * resident_ctas((const void*)k_scatter_levels, 128, 0, 16));
-        const int nl = c.n_levels;
-        auto level_rows = [&](int l) -> uint64_t {
-            const LevelDev& lv = ctx->enc.lv[l];
-            const uint64_t r = (uint64_t)lv.res + 1;
-            return lv.dense ? r * r * r : (uint64_t)ctx->enc.hash_mask + 1;
-        };
-        cudaError_t es = cudaSuccess;
-        for (int l0 = 0; l0 < nl && es == cudaSuccess;) {
-            const uint64_t row0 = ctx->enc.lv[l0].offset;
-            uint64_t row1 = row0 + level_rows(l0);
-            int l1 = l0 + 1;
-            while (l1 < nl && (ctx->enc.lv[l1].offset + level_rows(l1) - row0) * 8u <=
-                                  kScatterGroupBytes) {
-                row1 = ctx->enc.lv[l1].offset + level_rows(l1);
-                ++l1;
-            }
-            es = cudaMemsetAsync(ctx->grads + 2 * row0, 0, sizeof(float) * 2 * (row1 - row0), ss);
-            if (es != cudaSuccess) break;
-            sa.level_begin = (uint32_t)l0;
-            sa.level_end = (uint32_t)l1;
-            const uint32_t items = (uint32_t)(l1 - l0) * tiles;
-            const uint32_t g = g_max < items ? g_max : items;
-            ProfScope ps(ctx, NRRS_KERNEL_TRAIN_SCATTER, ss);
-            if (g) k_scatter_levels<<<g, 128, 0, ss>>>(sa);
-            es = cudaGetLastError();
-            l0 = l1;
-        }
-        return es;
+        return launch_scatter_table(ctx, v.pos, n,
+                                    LaneGrads{dxs, 2 * (size_t)n, 2, 1, a.inv_n}, ss);
     };
     bool forked = false;
     auto after_stat = [&]() -> cudaError_t {

@@ -68,6 +68,8 @@ struct InferArgs {
     unsigned long long* ext_acc;  // accumulate into this caller-owned sum instead (sharded)
     const uint8_t* enc_tiles;     // split mode: hash features per tile from k_encode_levels
     uint8_t* x1_tiles;            // split mode 2: RRSNet input per tile ([128 x 16], 4 KB)
+    const float* feat;            // FP32 path: the features of tiles tile_begin .. tile_end - 1
+    uint32_t tile_begin, tile_end;
 };
 
 // split inference mode: per tile, the 32 hash-grid features of its 128 vertices as a
@@ -84,6 +86,23 @@ struct EncodeLvArgs {
     uint32_t kdim;                // K of the tile layout: 32 (inference) or 64 (training input)
 };
 cudaError_t launch_encode_levels(const EncodeLvArgs& a, bool bf, int sm_count, cudaStream_t s);
+
+// the FP32 path's encoding: feature k of vertex m of tile t goes to
+// out[(t - tile_begin) * tile_stride + k * lane_stride + m], zeros past the end of a segment
+struct EncodeF32Args {
+    EncodeParams enc;
+    SegmentTable segs;
+    const float* pos;
+    const float* table;           // FP32 table [rows][2]
+    float* out;
+    size_t tile_stride, lane_stride;
+    uint32_t tile_begin, tile_end;
+};
+cudaError_t launch_encode_f32(const EncodeF32Args& a, int sm_count, cudaStream_t s);
+// FP32 inference runs in passes of at most this many tiles (1,048,576 vertices), whose features
+// are kTile x 32 floats each
+constexpr uint32_t kF32PassTiles = 8192;
+constexpr uint32_t kF32TileFloats = kTile * 32;
 
 // resident CTAs per SM of a kernel from its own resources (shared memory incl. the 1 KB the
 // runtime reserves per CTA, registers, warps), capped by `cap` (TMEM columns or a tuning choice)

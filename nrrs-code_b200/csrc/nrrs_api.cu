@@ -301,14 +301,35 @@ int run_infer(nrrs_ctx* ctx, const nrrs_vertex_soa* v, const SegmentTable& segs,
         ctx->last_infer_grid = g_last_grid;
         return NRRS_OK;
     }
-    {
-        ProfScope ps(ctx, c.precision == NRRS_PREC_FP32 ? NRRS_KERNEL_INFER_FP32 : NRRS_KERNEL_INFER_TC, s);
-        if (c.precision == NRRS_PREC_FP32)
+    if (c.precision == NRRS_PREC_FP32) {
+        // encoding and networks in passes that the feature scratch holds
+        EncodeF32Args ea{};
+        ea.enc = a.enc;
+        ea.segs = a.segs;
+        ea.pos = a.v.pos;
+        ea.table = a.table;
+        ea.out = ctx->feat;
+        ea.tile_stride = kF32TileFloats;
+        ea.lane_stride = kTile;
+        a.feat = ctx->feat;
+        for (uint32_t t0 = 0; t0 < segs.total_tiles; t0 += ctx->feat_tiles) {
+            a.tile_begin = ea.tile_begin = t0;
+            a.tile_end = ea.tile_end =
+                segs.total_tiles - t0 < ctx->feat_tiles ? segs.total_tiles : t0 + ctx->feat_tiles;
+            {
+                ProfScope ps(ctx, NRRS_KERNEL_ENCODE, s);
+                e = launch_encode_f32(ea, ctx->sm_count, s);
+            }
+            if (e != cudaSuccess) return cuda_fail(ctx, e, "encoding launch");
+            ProfScope ps(ctx, NRRS_KERNEL_INFER_FP32, s);
             e = launch_infer_fp32(a, c.statnet_width, c.statnet_hidden, c.rrsnet_width,
                                   c.rrsnet_hidden, ctx->sm_count, ctx->simt_ctas_per_sm, s);
-        else
-            e = launch_infer_tc(a, c.statnet_width, c.statnet_hidden, c.rrsnet_width, c.rrsnet_hidden,
-                                c.precision, ctx->sm_count, ctx->tc_ctas_per_sm, ctx->tc_wgs, 0, false, s);
+            if (e != cudaSuccess) return cuda_fail(ctx, e, "inference launch");
+        }
+    } else {
+        ProfScope ps(ctx, NRRS_KERNEL_INFER_TC, s);
+        e = launch_infer_tc(a, c.statnet_width, c.statnet_hidden, c.rrsnet_width, c.rrsnet_hidden,
+                            c.precision, ctx->sm_count, ctx->tc_ctas_per_sm, ctx->tc_wgs, 0, false, s);
     }
     if (e != cudaSuccess) return cuda_fail(ctx, e, "inference launch");
     ctx->last_infer_grid = g_last_grid;
@@ -575,7 +596,12 @@ int nrrs_create(const nrrs_config* cfg, nrrs_ctx** out) {
             return fail(nullptr, NRRS_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e)); \
         }                                                                              \
     } while (0)
-    NRRS_ALLOC(ctx->params, pb);
+    // FP32 contexts gather from the master table by 32-byte sectors: it starts 2 rows into its
+    // allocation where that puts the hashed levels on a sector and keeps the 16-byte alignment of
+    // the vectorised passes
+    if (c.precision == NRRS_PREC_FP32 && half_shift(ctx->enc) % 4 == 2) ctx->params_pad = 4;
+    NRRS_ALLOC(ctx->params, pb + sizeof(float) * ctx->params_pad);
+    ctx->params += ctx->params_pad;
     NRRS_ALLOC(ctx->grads, pb);
     NRRS_ALLOC(ctx->adam_m, pb);
     NRRS_ALLOC(ctx->adam_v, pb);
@@ -599,10 +625,17 @@ int nrrs_create(const nrrs_config* cfg, nrrs_ctx** out) {
     }
     if (c.ema_decay > 0.f) {
         NRRS_ALLOC(ctx->ema, pb);
-        NRRS_ALLOC(ctx->params_inf, pb);
+        NRRS_ALLOC(ctx->params_inf, pb + sizeof(float) * ctx->params_pad);
+        ctx->params_inf += ctx->params_pad;
         NRRS_ALLOC(ctx->wt_inf, sizeof(float) * ctx->wt_floats);
         if (ctx->table_h) NRRS_ALLOC(ctx->table_h_inf, half_table_bytes(ctx));
         if (ctx->cells) NRRS_ALLOC(ctx->cells_inf, 32 * (size_t)ctx->n_cells);
+    }
+    if (c.precision == NRRS_PREC_FP32) {
+        // a batched call's segments are padded to whole tiles
+        const uint32_t tiles = (c.max_queue + kTile - 1) / kTile + kMaxSegments;
+        ctx->feat_tiles = tiles < kF32PassTiles ? tiles : kF32PassTiles;
+        NRRS_ALLOC(ctx->feat, sizeof(float) * (size_t)kF32TileFloats * ctx->feat_tiles);
     }
     if (train_tc_supported(c))
         NRRS_ALLOC(ctx->tpack, train_pack_bytes(c.statnet_width, c.statnet_hidden,
@@ -671,14 +704,14 @@ void nrrs_destroy(nrrs_ctx* ctx) {
     }
     if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
     if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
-    cudaFree(ctx->params);
+    if (ctx->params) cudaFree(ctx->params - ctx->params_pad);
     cudaFree(ctx->grads);
     cudaFree(ctx->adam_m);
     cudaFree(ctx->adam_v);
     cudaFree(ctx->table_h);
     cudaFree(ctx->cells);
     cudaFree(ctx->ema);
-    cudaFree(ctx->params_inf);
+    if (ctx->params_inf) cudaFree(ctx->params_inf - ctx->params_pad);
     cudaFree(ctx->wt_inf);
     cudaFree(ctx->table_h_inf);
     cudaFree(ctx->cells_inf);
@@ -687,6 +720,7 @@ void nrrs_destroy(nrrs_ctx* ctx) {
     cudaFree(ctx->wpack);
     cudaFree(ctx->tpack);
     cudaFree(ctx->enc_tiles);
+    cudaFree(ctx->feat);
     cudaFree(ctx->x1_tiles);
     cudaFree(ctx->scr);
     cudaFree(ctx->split_tmp);
