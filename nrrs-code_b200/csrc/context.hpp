@@ -78,7 +78,7 @@ struct nrrs_ctx {
     void* train_scratch = nullptr;
     size_t train_scratch_bytes = 0;
     double* loss_dev = nullptr;  // [2] last losses
-    double* loss_sums = nullptr; // [4] batch sums of the loss weights (nrrs_train_step_batch)
+    double* loss_sums = nullptr; // batch sums of the loss weights (launch_loss_sums' block)
 
     int last_infer_grid = 0;
     int tc_ctas_per_sm = 0;      // autotuned occupancy of the tcgen05 kernel (0 = default)
@@ -134,7 +134,10 @@ inline EncodeParams half_enc(const nrrs_ctx* ctx) {
 int train_step_impl(nrrs_ctx* ctx, const VertexPtrs& v, const float* target, uint32_t n,
                     double* loss_dev, cudaStream_t s, bool apply = true,
                     const LossWeights* lw = nullptr);
-// batch sums of the loss weights into out[3] (sum s, sum w, mean pixel error)
+// batch sums of the loss weights into out[3] (sum s, sum w, mean pixel error); out is a block of
+// kLossSumDoubles, zeroed once
+constexpr uint32_t kLossSumBlocks = 128;
+constexpr uint32_t kLossSumDoubles = 4 + 2 * kLossSumBlocks + 1;
 cudaError_t launch_loss_sums(const LossWeights& w, uint32_t n, const float* error_sum,
                              uint32_t n_pixels, double* out, cudaStream_t s);
 // The table gradient of an n-sample step from its lane gradients, added to zeroed slices of

@@ -107,7 +107,7 @@ __device__ __forceinline__ void fwd_layer(const float* __restrict__ wt, int k_ef
             if (store) {
                 float* g = scr + (size_t)(row0 + n) * ld + i0 + m0;
                 *reinterpret_cast<float4*>(g) = make_float4(r[0], r[1], r[2], r[3]);
-                *reinterpret_cast<float4*>(g + 4) = make_float4(r[4], r[5], r[6], r[7]);
+                *reinterpret_cast<float4*>(g + 32) = make_float4(r[4], r[5], r[6], r[7]);
             }
         });
     pos = bits;
@@ -130,7 +130,7 @@ __device__ __forceinline__ void bwd_layer(const float* __restrict__ w, float* ti
             simt::tile_store8(tile, n, m0, r);
             float* g = scr + (size_t)(out0 + n) * ld + i0 + m0;
             *reinterpret_cast<float4*>(g) = make_float4(r[0], r[1], r[2], r[3]);
-            *reinterpret_cast<float4*>(g + 4) = make_float4(r[4], r[5], r[6], r[7]);
+            *reinterpret_cast<float4*>(g + 32) = make_float4(r[4], r[5], r[6], r[7]);
         });
 }
 
@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(TrShape<WS>::kThr, WS == 128 ? 4 : 8)
             if (n >= HL) return;
             float* g = scr + (size_t)(a.r_dx + n) * ld + i0 + m0;
             *reinterpret_cast<float4*>(g) = make_float4(v[0], v[1], v[2], v[3]);
-            *reinterpret_cast<float4*>(g + 4) = make_float4(v[4], v[5], v[6], v[7]);
+            *reinterpret_cast<float4*>(g + 32) = make_float4(v[4], v[5], v[6], v[7]);
         });
 
         // ---- glue and the RRSNet forward for the batch sums ----
@@ -444,33 +444,58 @@ __global__ void __launch_bounds__(TrShape<WR>::kThr, WR == 128 ? 4 : 8)
     }
 }
 
-// ---- batch sums of the loss weights (one block, fixed order: deterministic) ----
+// ---- batch sums of the loss weights (fixed slices and order: deterministic) ----
 // out[0] = sum s_i, out[1] = sum w_i, out[2] = the mean pixel error error_sum / n_pixels (1 when
-// no error sum is given)
-__global__ void __launch_bounds__(1024) k_loss_sums(const __grid_constant__ LossWeights w,
-                                                   uint32_t n, const float* error_sum,
-                                                   uint32_t n_pixels, double* out) {
-    __shared__ double red[2][32];
+// no error sum is given). kSumBlocks CTAs each sum a fixed slice into part[b]; the last one to
+// finish (a counter, which it resets) adds the slices in order. One CTA for the whole batch took
+// 28 us at 50,021 samples; this takes 4.9.
+constexpr int kSumThr = 512;
+__global__ void __launch_bounds__(kSumThr) k_loss_sums(const __grid_constant__ LossWeights w,
+                                                       uint32_t n, const float* error_sum,
+                                                       uint32_t n_pixels, double* out, double* part,
+                                                       unsigned* done) {
+    __shared__ double red[2][kSumThr / 32];
+    __shared__ bool s_last;
+    const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+    auto block_pair = [&](double& s, double& ww) {   // sums over the CTA, valid on thread 0
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            s += __shfl_xor_sync(0xffffffffu, s, o);
+            ww += __shfl_xor_sync(0xffffffffu, ww, o);
+        }
+        if (lane == 0) red[0][wid] = s, red[1][wid] = ww;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            s = ww = 0.0;
+            for (int k = 0; k < kSumThr / 32; ++k) s += red[0][k], ww += red[1][k];
+        }
+    };
     double s = 0.0, ww = 0.0;
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+    for (uint32_t i = blockIdx.x * kSumThr + threadIdx.x; i < n; i += gridDim.x * kSumThr) {
         s += (double)loss_w_stat(w, i);
         ww += (double)loss_w_rrs(w, i);
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        s += __shfl_xor_sync(0xffffffffu, s, o);
-        ww += __shfl_xor_sync(0xffffffffu, ww, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        red[0][threadIdx.x >> 5] = s;
-        red[1][threadIdx.x >> 5] = ww;
+    block_pair(s, ww);
+    if (threadIdx.x == 0) {
+        part[2 * blockIdx.x] = s;
+        part[2 * blockIdx.x + 1] = ww;
+        __threadfence();
+        s_last = atomicAdd(done, 1u) == gridDim.x - 1;
     }
     __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    s = ww = 0.0;
+    for (uint32_t b = threadIdx.x; b < gridDim.x; b += kSumThr) {
+        s += __ldcg(part + 2 * b);
+        ww += __ldcg(part + 2 * b + 1);
+    }
+    __syncthreads();
+    block_pair(s, ww);
     if (threadIdx.x == 0) {
-        double ts = 0.0, tw = 0.0;
-        for (int k = 0; k < (int)(blockDim.x >> 5); ++k) ts += red[0][k], tw += red[1][k];
-        out[0] = ts;
-        out[1] = tw;
+        *done = 0;
+        out[0] = s;
+        out[1] = ww;
         double em = 1.0;
         if (error_sum && n_pixels) {
             em = (double)*error_sum / (double)n_pixels;
@@ -484,7 +509,11 @@ __global__ void __launch_bounds__(1024) k_loss_sums(const __grid_constant__ Loss
 
 cudaError_t launch_loss_sums(const LossWeights& w, uint32_t n, const float* error_sum,
                              uint32_t n_pixels, double* out, cudaStream_t s) {
-    k_loss_sums<<<1, 1024, 0, s>>>(w, n, error_sum, n_pixels, out);
+    // out[4] on: a pair per CTA, then the counter
+    const uint32_t need = (n + kSumThr - 1) / kSumThr;
+    k_loss_sums<<<need < kLossSumBlocks ? need : kLossSumBlocks, kSumThr, 0, s>>>(
+        w, n, error_sum, n_pixels, out, out + 4,
+        reinterpret_cast<unsigned*>(out + 4 + 2 * kLossSumBlocks));
     return cudaGetLastError();
 }
 
@@ -546,22 +575,27 @@ __device__ __forceinline__ void wgrad_tile(const WGradArgs& a, const WJob& j, fl
                 make_float4(0.f, 0.f, 0.f, 0.f);
     }
     const uint32_t stages = (i1 - i0 + kWS - 1) / kWS;
+    // a thread copies the same 16 bytes of rows r0, r0 + 16, .. in every stage
+    const int r0 = tid / (kWS / 4), q0 = 4 * (tid % (kWS / 4));
+    constexpr int kStep = kWThr / (kWS / 4);
+    const float* gd = a.act + (size_t)(j.d_row + r0) * a.ld + i0 + q0;
+    const float* ga = a.act + (size_t)(j.a_row + r0) * a.ld + i0 + q0;
+    const size_t gstep = (size_t)kStep * a.ld;
     auto issue = [&](uint32_t s) {
         if (s < stages) {
-            float* dst = sm + (s % kWStages) * kStage;
-            const uint32_t ib = i0 + s * kWS;
-            for (int e = tid; e < ROWS * (kWS / 4); e += kWThr) {
-                const int r = e / (kWS / 4), q = e % (kWS / 4);
-                const bool d = r < TM;
-                const uint32_t rr = d ? (uint32_t)r : (uint32_t)(r - TM);
-                if (rr >= (d ? j.M : j.N)) continue;
-                const uint32_t i = ib + 4 * q;
-                const uint32_t left = i < i1 ? i1 - i : 0u;
-                simt::cp_async16_n(dst + r * kWPitch + 4 * q,
-                                   a.act + (size_t)((d ? j.d_row : j.a_row) + rr) * a.ld +
-                                       (left ? i : i0),
-                                   left >= 4u ? 16u : 4u * left);
-            }
+            float* dst = sm + (s % kWStages) * kStage + r0 * kWPitch + q0;
+            const uint32_t i = i0 + s * kWS + q0;
+            const uint32_t left = i < i1 ? i1 - i : 0u;
+            const uint32_t bytes = left >= 4u ? 16u : 4u * left;
+            const size_t o = left ? s * kWS : 0;     // nothing left: any valid address
+#pragma unroll
+            for (int k = 0; k < (TM + kStep - 1) / kStep; ++k)
+                if ((uint32_t)(r0 + k * kStep) < j.M)
+                    simt::cp_async16_n(dst + k * kStep * kWPitch, gd + k * gstep + o, bytes);
+#pragma unroll
+            for (int k = 0; k < (TN + kStep - 1) / kStep; ++k)
+                if ((uint32_t)(r0 + k * kStep) < j.N)
+                    simt::cp_async16_n(dst + (TM + k * kStep) * kWPitch, ga + k * gstep + o, bytes);
         }
         simt::cp_async_commit();
     };
@@ -626,9 +660,11 @@ constexpr WShape kWShapes[] = {{64, 64}, {32, 32}, {64, 16}, {32, 16}, {8, 64}, 
 // operands are read once per output tile). 64 x 64 tiles of 8 x 4 outputs per thread read 12
 // 16-byte words per 128 FMAs; two CTAs per SM. The tile follows the layer (32 x 32 for the shipped
 // network, 8 rows for the output layers), so little work is done for padding. Measured: 64 x 2,
-// 262,144 samples 272 us, where 16 outputs per thread fed by scalar shared-memory reads, one
-// stage deep, took 937 us; shipped network, 50,021 samples 44 us against 419 us (25 chunks of
-// 2,048 left the chip idle).
+// 262,144 samples 251 us (272 with a stage's copy addresses formed by divisions each time),
+// where 16 outputs per thread fed by scalar shared-memory reads, one stage deep, took 937 us;
+// shipped network, 50,021 samples 38 us against 419 us (25 chunks of 2,048 left the chip idle).
+// The tile loop alone, on resident shared memory, reaches 46 TFLOP/s (43 to 49 for 4 x 4 to 8 x 8
+// outputs per thread, paired or not); the work here is 7.5 GFLOP.
 __global__ void __launch_bounds__(kWThr, 2) k_wgrad(const __grid_constant__ WGradArgs a) {
     extern __shared__ float4 smem4[];
     float* sm = reinterpret_cast<float*>(smem4);

@@ -646,7 +646,7 @@ int nrrs_create(const nrrs_config* cfg, nrrs_ctx** out) {
     NRRS_ALLOC(ctx->split_tmp, (size_t)ctx->max_chunks * kDecChunk);
     NRRS_ALLOC(ctx->loss_dev, sizeof(double) * 2);
     NRRS_ALLOC(ctx->segs_dev, sizeof(SegmentTable) * 2);
-    NRRS_ALLOC(ctx->loss_sums, sizeof(double) * 4);
+    NRRS_ALLOC(ctx->loss_sums, sizeof(double) * kLossSumDoubles);
     ctx->train_scratch_bytes = train_scratch_bytes(c, c.max_train, ctx->sm_count);
     NRRS_ALLOC(ctx->train_scratch, ctx->train_scratch_bytes);
 #undef NRRS_ALLOC
@@ -673,6 +673,7 @@ int nrrs_create(const nrrs_config* cfg, nrrs_ctx** out) {
         e = cudaMemcpy(&ctx->scr->epoch, &one, sizeof(one), cudaMemcpyHostToDevice);
     }
     if (e == cudaSuccess) e = cudaMemset(ctx->loss_dev, 0, sizeof(double) * 2);
+    if (e == cudaSuccess) e = cudaMemset(ctx->loss_sums, 0, sizeof(double) * kLossSumDoubles);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming);

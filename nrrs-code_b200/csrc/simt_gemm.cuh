@@ -78,8 +78,10 @@ __device__ __forceinline__ void load_chunk(float* dst, const float* __restrict__
         cp_async16(dst + 4 * q, src + (size_t)(q / (W / 4)) * ldb + 4 * (q % (W / 4)));
 }
 
-// out[n][m] = epi(j, n, m0, v[8]) with v[i] = sum_{k < k_eff} B[k][n] act[k][m0 + i], for the 8
-// samples m0 .. m0+7 and the C neurons n each thread owns (j = 0 .. C-1 counts them). Every read
+// out[n][m] = epi(j, n, m0, v[8]) with v[i] = sum_{k < k_eff} B[k][n] act[k][m] for the 8 samples
+// m = m0 .. m0+3 and m0+32 .. m0+35 and the C neurons n each thread owns (j = 0 .. C-1 counts
+// them). Four samples each from both halves: the threads of a warp that share a neuron then hold
+// 64 consecutive bytes, whole sectors when they store to global memory. Every read
 // of the tile ends at the chunk loop's last barrier, so epi may overwrite it in place; a barrier
 // follows epi. wch holds two chunks of kKC x W floats.
 template <int W, int NT, class Epi>
@@ -89,7 +91,7 @@ __device__ __forceinline__ void tile_gemm(const float* __restrict__ B, int ldb, 
     constexpr int TX = W / C;
     constexpr int CW = C < 4 ? C : 4;         // consecutive neurons of a thread's group
     static_assert(C == 2 || C == 4 || C == 8, "tile widths");
-    const int tx = tid % TX, ty = tid / TX;   // ty 0..7: samples ty*8 .. +7
+    const int tx = tid % TX, ty = tid / TX;   // ty 0..7: samples 4 ty .. +3 and 32 + 4 ty .. +3
     unsigned long long acc[4][C];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -113,9 +115,9 @@ __device__ __forceinline__ void tile_gemm(const float* __restrict__ B, int ldb, 
         auto step = [&](int kk) {
             const int sw = (c * kKC + kk) & 28;
             const ulonglong2 a0 =
-                *reinterpret_cast<const ulonglong2*>(A + kk * kTM + ((ty * 8) ^ sw));
+                *reinterpret_cast<const ulonglong2*>(A + kk * kTM + ((ty * 4) ^ sw));
             const ulonglong2 a1 =
-                *reinterpret_cast<const ulonglong2*>(A + kk * kTM + ((ty * 8 + 4) ^ sw));
+                *reinterpret_cast<const ulonglong2*>(A + kk * kTM + 32 + ((ty * 4) ^ sw));
             const unsigned long long av[4] = {a0.x, a0.y, a1.x, a1.y};
             float bv[C];
             if constexpr (C == 2) {
@@ -151,15 +153,15 @@ __device__ __forceinline__ void tile_gemm(const float* __restrict__ B, int ldb, 
         float v[8];
 #pragma unroll
         for (int i = 0; i < 4; ++i) unpack2f(acc[i][j], v[2 * i], v[2 * i + 1]);
-        epi(j, n, ty * 8, v);
+        epi(j, n, ty * 4, v);
     }
     __syncthreads();
 }
 
-// 8 consecutive values of tile row n from samples m0 .. m0+7
+// 8 values of tile row n: samples m0 .. m0+3 and m0+32 .. m0+35
 __device__ __forceinline__ void tile_store8(float* act, int n, int m0, const float* v) {
     *reinterpret_cast<float4*>(act + at(n, m0)) = make_float4(v[0], v[1], v[2], v[3]);
-    *reinterpret_cast<float4*>(act + at(n, m0 + 4)) = make_float4(v[4], v[5], v[6], v[7]);
+    *reinterpret_cast<float4*>(act + at(n, m0 + 32)) = make_float4(v[4], v[5], v[6], v[7]);
 }
 
 // y[o] = sum_k wt[k][o] tile[k][m] for a narrow output layer (wt is [W][OUT rounded up to 4]), k
