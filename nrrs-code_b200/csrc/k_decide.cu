@@ -10,14 +10,18 @@
 // them does not change a bit (the reference's FP32 sum depends on the occupancy-chosen grid).
 // Two emissions give the same queue, in vertex order with the s copies of a vertex contiguous,
 // over 2048-vertex chunks:
-//  * the context path runs two passes (k_decide_count, k_decide_emit): decide and count every
-//    chunk, scan the chunk totals in the count pass's last CTA, then emit each chunk at its
-//    prefix from its split counts. No CTA waits on another (4K bounce: 0.063 ms against
-//    0.098 ms for the single pass, whose CTAs spent most of their time at block barriers);
+//  * the context path decides a single segment of up to 65,536 vertices in one cluster
+//    (k_decide_small) and runs two passes otherwise (k_decide_count, k_decide_emit): decide and
+//    count every chunk, scan the chunk totals in the count pass's last CTA, then emit each chunk
+//    at its prefix from its split counts. No CTA spins on another (4K bounce: 0.063 ms against
+//    0.098 ms for the single pass, whose CTAs spent most of their time at block barriers). These
+//    kernels are set up while the one before them finishes (programmatic stream serialisation);
 //  * the allocation-free entry point keeps the single-pass prefix sum with decoupled look-back
 //    (k_decide), which needs no per-vertex scratch: chunks are taken in ticket order, so every
 //    predecessor of a waiting chunk has already started and the wait ends; each wait is bounded
 //    and reports NRRS_DEV_TIMEOUT. One warp reads 32 predecessor states at a time.
+#include <cooperative_groups.h>
+
 #include "kernels.hpp"
 
 namespace nrrs {
@@ -325,13 +329,88 @@ __device__ __forceinline__ uint8_t* split_of_chunk(const DecideArgs& a, unsigned
     return a.split_chunked ? a.split + (size_t)c * kDecChunk : a.split + first;
 }
 
+// Decision of the kDecVPT consecutive vertices v0 .. (those below `end`) of segment sg: rrs_norm,
+// and the split counts into sv and, where cs is not null, to cs[0 ..]. Returns their sum.
+__device__ __forceinline__ unsigned decide_run(const DecideArgs& a, float scale, unsigned v0,
+                                               unsigned end, uint8_t* cs, unsigned (&sv)[kDecVPT],
+                                               unsigned* flags) {
+    const bool vec = v0 + kDecVPT <= end &&
+                     ((reinterpret_cast<uintptr_t>(a.rrs + v0) |
+                       reinterpret_cast<uintptr_t>(a.rnd + v0)) & 15u) == 0;
+    constexpr int kQ = kDecVPT / 4;
+    float rv[kDecVPT], nv[kDecVPT];
+    if (vec) {
+#pragma unroll
+        for (int g = 0; g < kQ; ++g) {
+            const float4 r4 = *reinterpret_cast<const float4*>(a.rrs + v0 + 4 * g);
+            const float4 n4 = *reinterpret_cast<const float4*>(a.rnd + v0 + 4 * g);
+            rv[4 * g] = r4.x; rv[4 * g + 1] = r4.y; rv[4 * g + 2] = r4.z; rv[4 * g + 3] = r4.w;
+            nv[4 * g] = n4.x; nv[4 * g + 1] = n4.y; nv[4 * g + 2] = n4.z; nv[4 * g + 3] = n4.w;
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < kDecVPT; ++j) {
+            rv[j] = v0 + j < end ? a.rrs[v0 + j] : 0.f;
+            nv[j] = v0 + j < end ? a.rnd[v0 + j] : 0.f;
+        }
+    }
+    float rn[kDecVPT];
+    unsigned local = 0;
+#pragma unroll
+    for (int j = 0; j < kDecVPT; ++j) {
+        const unsigned v = v0 + j;
+        rn[j] = 0.f;
+        sv[j] = 0u;
+        if (v < end) {
+            const float r = __fmul_rn(rv[j], scale);
+            rn[j] = r;
+            if (a.rrs_norm && (a.sidx || !vec)) a.rrs_norm[a.sidx ? a.sidx[v] : v] = r;
+            sv[j] = split_count(r, nv[j], flags);
+            if (cs && !vec) cs[j] = (uint8_t)sv[j];
+            local += sv[j];
+        }
+    }
+    if (vec) {
+        if (a.rrs_norm && !a.sidx && (reinterpret_cast<uintptr_t>(a.rrs_norm + v0) & 15u) == 0) {
+#pragma unroll
+            for (int g = 0; g < kQ; ++g)
+                *reinterpret_cast<float4*>(a.rrs_norm + v0 + 4 * g) =
+                    make_float4(rn[4 * g], rn[4 * g + 1], rn[4 * g + 2], rn[4 * g + 3]);
+        } else if (a.rrs_norm && !a.sidx) {
+#pragma unroll
+            for (int j = 0; j < kDecVPT; ++j) a.rrs_norm[v0 + j] = rn[j];
+        }
+        if (cs && (reinterpret_cast<uintptr_t>(cs) & 3u) == 0) {
+#pragma unroll
+            for (int g = 0; g < kQ; ++g)
+                reinterpret_cast<uint32_t*>(cs)[g] = sv[4 * g] | sv[4 * g + 1] << 8 |
+                                                     sv[4 * g + 2] << 16 | sv[4 * g + 3] << 24;
+        } else if (cs) {
+#pragma unroll
+            for (int j = 0; j < kDecVPT; ++j) cs[j] = (uint8_t)sv[j];
+        }
+    }
+    return local;
+}
+
+// waits for the kernels before this one in its stream (and has their writes visible); a kernel
+// launched with programmatic stream serialisation calls it before it touches memory
+__device__ __forceinline__ void wait_for_stream() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// lets the next kernel of the stream be set up while this one finishes
+__device__ __forceinline__ void let_next_start() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __global__ void __launch_bounds__(kDecThreads) k_decide_count(const __grid_constant__ DecideArgs a) {
     __shared__ unsigned s_red[kDecThreads / 32];
     __shared__ int s_last;
-    __shared__ unsigned long long s_scan[kDecThreads];
+    __shared__ unsigned long long s_scan[kDecThreads / 32];
     const int tid = threadIdx.x;
     const unsigned c = blockIdx.x;
     unsigned flags = 0;
+    wait_for_stream();
     const SegmentTable& S = seg_table(a.segs);
     unsigned local = 0;
     if (c < S.total_tiles) {
@@ -340,64 +419,10 @@ __global__ void __launch_bounds__(kDecThreads) k_decide_count(const __grid_const
         const unsigned lc = c - sg.tile_start;
         const unsigned end = sg.offset + min(sg.count, (lc + 1) * kDecChunk);
         const float scale = decide_scale(a, sg, si);
-        const unsigned v0 = sg.offset + lc * kDecChunk + tid * kDecVPT;
-        uint8_t* cs = split_of_chunk(a, c, sg.offset + lc * kDecChunk) + tid * kDecVPT;
-        const bool vec = v0 + kDecVPT <= end &&
-                         ((reinterpret_cast<uintptr_t>(a.rrs + v0) |
-                           reinterpret_cast<uintptr_t>(a.rnd + v0)) & 15u) == 0;
-        constexpr int kQ = kDecVPT / 4;
-        float rv[kDecVPT], nv[kDecVPT];
-        if (vec) {
-#pragma unroll
-            for (int g = 0; g < kQ; ++g) {
-                const float4 r4 = *reinterpret_cast<const float4*>(a.rrs + v0 + 4 * g);
-                const float4 n4 = *reinterpret_cast<const float4*>(a.rnd + v0 + 4 * g);
-                rv[4 * g] = r4.x; rv[4 * g + 1] = r4.y; rv[4 * g + 2] = r4.z; rv[4 * g + 3] = r4.w;
-                nv[4 * g] = n4.x; nv[4 * g + 1] = n4.y; nv[4 * g + 2] = n4.z; nv[4 * g + 3] = n4.w;
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < kDecVPT; ++j) {
-                rv[j] = v0 + j < end ? a.rrs[v0 + j] : 0.f;
-                nv[j] = v0 + j < end ? a.rnd[v0 + j] : 0.f;
-            }
-        }
-        float rn[kDecVPT];
-        uint32_t sp[kQ];
-#pragma unroll
-        for (int g = 0; g < kQ; ++g) sp[g] = 0u;
-#pragma unroll
-        for (int j = 0; j < kDecVPT; ++j) {
-            const unsigned v = v0 + j;
-            rn[j] = 0.f;
-            if (v < end) {
-                const float r = __fmul_rn(rv[j], scale);
-                rn[j] = r;
-                if (a.rrs_norm && (a.sidx || !vec)) a.rrs_norm[a.sidx ? a.sidx[v] : v] = r;
-                const unsigned s = split_count(r, nv[j], &flags);
-                if (!vec) cs[j] = (uint8_t)s;
-                sp[j >> 2] |= s << (8 * (j & 3));
-                local += s;
-            }
-        }
-        if (vec) {
-            if (a.rrs_norm && !a.sidx && (reinterpret_cast<uintptr_t>(a.rrs_norm + v0) & 15u) == 0) {
-#pragma unroll
-                for (int g = 0; g < kQ; ++g)
-                    *reinterpret_cast<float4*>(a.rrs_norm + v0 + 4 * g) =
-                        make_float4(rn[4 * g], rn[4 * g + 1], rn[4 * g + 2], rn[4 * g + 3]);
-            } else if (a.rrs_norm && !a.sidx) {
-#pragma unroll
-                for (int j = 0; j < kDecVPT; ++j) a.rrs_norm[v0 + j] = rn[j];
-            }
-            if ((reinterpret_cast<uintptr_t>(cs) & 3u) == 0) {
-#pragma unroll
-                for (int g = 0; g < kQ; ++g) reinterpret_cast<uint32_t*>(cs)[g] = sp[g];
-            } else {
-#pragma unroll
-                for (int j = 0; j < kDecVPT; ++j) cs[j] = (uint8_t)(sp[j >> 2] >> (8 * (j & 3)));
-            }
-        }
+        const unsigned first = sg.offset + lc * kDecChunk;
+        unsigned sv[kDecVPT];
+        local = decide_run(a, scale, first + tid * kDecVPT, end,
+                           split_of_chunk(a, c, first) + tid * kDecVPT, sv, &flags);
     }
     // chunk total (split counts are at most 255, 2,048 per chunk: no overflow)
     const unsigned total = block_sum_u(local, s_red);
@@ -407,56 +432,61 @@ __global__ void __launch_bounds__(kDecThreads) k_decide_count(const __grid_const
         __threadfence();
         s_last = atomicAdd(&a.scr->done, 1u) == gridDim.x - 1;
     }
+    let_next_start();
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    // the last CTA: exclusive prefix of the chunk totals per segment, saturating like the
-    // single-pass kernel; thread t scans a contiguous run of each segment's chunks
-    for (int k = 0; k < S.n; ++k) {
-        const Segment& sg = S.s[k];
-        const unsigned nch = (sg.count + kDecChunk - 1) / kDecChunk;
-        const unsigned per = (nch + kDecThreads - 1) / kDecThreads;
-        const unsigned lo = sg.tile_start + min(nch, tid * per);
-        const unsigned hi = sg.tile_start + min(nch, (tid + 1) * per);
-        // the totals come in batches of independent L2 loads (the other CTAs' stores are visible
-        // after their fences and the done counter)
-        unsigned long long mine = 0;
-        for (unsigned q0 = lo; q0 < hi; q0 += 8) {
-            unsigned t8[8];
+    // The last CTA turns the totals into exclusive 64-bit prefixes over the chunks of all segments
+    // (a segment's own prefix is the difference to its first chunk's): thread t scans a contiguous
+    // run, in batches of independent L2 loads (the other CTAs' stores are visible after their
+    // fences and the done counter). One scan for all segments: a scan per segment, 16 block
+    // barriers each, made a 10-segment count 50 us instead of 38 (5,925,732 vertices).
+    const int lane = tid & 31, wid = tid >> 5;
+    const unsigned n = S.total_tiles;
+    const unsigned per = (n + kDecThreads - 1) / kDecThreads;
+    const unsigned lo = min(n, tid * per), hi = min(n, (tid + 1) * per);
+    unsigned long long mine = 0;
+    for (unsigned q0 = lo; q0 < hi; q0 += 8) {
+        unsigned t8[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) t8[j] = q0 + j < hi ? (unsigned)__ldcg(&a.states[q0 + j]) : 0u;
+        for (int j = 0; j < 8; ++j) t8[j] = q0 + j < hi ? (unsigned)__ldcg(&a.states[q0 + j]) : 0u;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) mine += t8[j];
-        }
-        s_scan[tid] = mine;
-        __syncthreads();
-#pragma unroll 1
-        for (int o = 1; o < kDecThreads; o <<= 1) {
-            const unsigned long long y = tid >= o ? s_scan[tid - o] : 0ull;
-            __syncthreads();
-            s_scan[tid] += y;
-            __syncthreads();
-        }
-        unsigned long long run = tid ? s_scan[tid - 1] : 0ull;
-        for (unsigned q0 = lo; q0 < hi; q0 += 8) {
-            unsigned t8[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) t8[j] = q0 + j < hi ? (unsigned)__ldcg(&a.states[q0 + j]) : 0u;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                if (q0 + j < hi) __stcg(&a.states[q0 + j], run > 0xffffffffull ? 0xffffffffull : run);
-                run += t8[j];
-            }
-        }
-        if (tid == kDecThreads - 1) {
-            const unsigned long long tot = s_scan[tid];
-            a.next_size[k] = tot > 0xffffffffull ? 0xffffffffu : (unsigned)tot;
-        }
-        __syncthreads();
+        for (int j = 0; j < 8; ++j) mine += t8[j];
     }
-    // restore the scratch for the next launch
+    unsigned long long incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) s_scan[wid] = incl;
+    __syncthreads();
+    unsigned long long run = incl - mine, all = 0;
+#pragma unroll
+    for (int k = 0; k < kDecThreads / 32; ++k) {
+        if (k < wid) run += s_scan[k];
+        all += s_scan[k];
+    }
+    for (unsigned q0 = lo; q0 < hi; q0 += 8) {
+        unsigned t8[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) t8[j] = q0 + j < hi ? (unsigned)__ldcg(&a.states[q0 + j]) : 0u;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (q0 + j < hi) __stcg(&a.states[q0 + j], run);
+            run += t8[j];
+        }
+    }
+    __syncthreads();
+    if (tid < S.n) {
+        const Segment& sg = S.s[tid];
+        const unsigned b = sg.tile_start, e = b + (sg.count + kDecChunk - 1) / kDecChunk;
+        const unsigned long long tot = (e < n ? __ldcg(&a.states[e]) : all) -
+                                       (b < n ? __ldcg(&a.states[b]) : all);
+        a.next_size[tid] = tot > 0xffffffffull ? 0xffffffffu : (unsigned)tot;
+        a.scr->sum_acc[tid] = 0ull;   // restore the scratch for the next launch
+    }
     if (tid == 0) {
-        for (int k = 0; k < S.n; ++k) a.scr->sum_acc[k] = 0ull;
         a.scr->ticket = 0;
         a.scr->done = 0;
         a.scr->epoch = a.scr->epoch + 1;
@@ -471,6 +501,7 @@ __global__ void __launch_bounds__(kDecThreads) k_decide_emit(const __grid_consta
     __shared__ unsigned s_warp[kDecThreads / 32];
     const int tid = threadIdx.x;
     const unsigned c = blockIdx.x;
+    wait_for_stream();
     const SegmentTable& S = seg_table(a.segs);
     if (c >= S.total_tiles) return;
     unsigned flags = 0;
@@ -479,7 +510,8 @@ __global__ void __launch_bounds__(kDecThreads) k_decide_emit(const __grid_consta
     const unsigned lc = c - sg.tile_start;
     const unsigned end = sg.offset + min(sg.count, (lc + 1) * kDecChunk);
     const unsigned v0 = sg.offset + lc * kDecChunk + tid * kDecVPT;
-    const unsigned prefix = (unsigned)a.states[c];
+    const unsigned long long in_seg = a.states[c] - a.states[sg.tile_start];
+    const unsigned prefix = in_seg > 0xffffffffull ? 0xffffffffu : (unsigned)in_seg;
     const uint8_t* cs = split_of_chunk(a, c, sg.offset + lc * kDecChunk) + tid * kDecVPT;
     unsigned sv[kDecVPT];
     unsigned local = 0;
@@ -541,6 +573,86 @@ __global__ void __launch_bounds__(kDecThreads) k_decide_emit(const __grid_consta
                 else flags |= NRRS_DEV_OVERFLOW;
             }
         }
+    }
+    if (flags) atomicOr(&a.scr->status, flags);
+}
+
+// The whole decision of one segment of up to kSmallSpan x 8 vertices as one cluster of up to 8 CTAs:
+// decide, scan in the CTA, exchange the CTA totals through distributed shared memory, emit. Two
+// grids (count, emission) are launch and memory latencies at this size: 3,071 vertices 7.0 us
+// against 7.1 + 3.7 and a gap, 65,536 vertices 7.6 against 7.4 + 3.5. A cluster of 8 is the largest
+// portable one, which sets the bound of 65,536 vertices.
+constexpr unsigned kSmallThreads = 1024;
+constexpr unsigned kSmallSpan = kSmallThreads * kDecVPT;   // vertices per CTA: 8,192
+constexpr unsigned kSmallStage = 10240;                    // E[s] is about 1
+
+__global__ void __launch_bounds__(kSmallThreads) k_decide_small(const __grid_constant__ DecideArgs a) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    __shared__ uint32_t s_stage[kSmallStage];
+    __shared__ unsigned s_warp[kSmallThreads / 32];
+    __shared__ unsigned s_tot[8];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const unsigned rank = blockIdx.x;
+    unsigned flags = 0;
+    wait_for_stream();
+    const SegmentTable& S = seg_table(a.segs);
+    const Segment& sg = S.s[0];
+    const unsigned end = sg.offset + min(sg.count, (rank + 1) * kSmallSpan);
+    const unsigned v0 = sg.offset + rank * kSmallSpan + tid * kDecVPT;
+    const float scale = decide_scale(a, sg, 0);
+    unsigned sv[kDecVPT];
+    const unsigned local =
+        decide_run(a, scale, v0, end, a.split_chunked ? nullptr : a.split + v0, sv, &flags);
+    unsigned incl = local;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) s_warp[wid] = incl;
+    __syncthreads();
+    if (wid == 0) {
+        unsigned w = s_warp[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned y = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += y;
+        }
+        s_warp[lane] = w;
+        const unsigned total = __shfl_sync(0xffffffffu, w, 31);
+        if ((unsigned)lane < gridDim.x) *cluster.map_shared_rank(&s_tot[rank], lane) = total;
+    }
+    cluster.sync();   // every CTA has every total, and has read the sum
+    unsigned prefix = 0;
+    for (unsigned r = 0; r < rank; ++r) prefix += s_tot[r];   // at most 65,536 x 255 entries
+    const unsigned thread_excl = (wid ? s_warp[wid - 1] : 0) + incl - local;
+    const unsigned total = s_warp[kSmallThreads / 32 - 1];
+    if (tid == 0 && rank == gridDim.x - 1) a.next_size[0] = prefix + total;
+    if (tid == 0 && rank == 0) a.scr->sum_acc[0] = 0ull;   // restore the scratch
+
+    uint32_t* q = a.queue + sg.queue_offset + prefix;
+    const unsigned room = prefix < sg.queue_capacity ? sg.queue_capacity - prefix : 0u;
+    unsigned pos = thread_excl;
+    if (total <= kSmallStage) {
+#pragma unroll
+        for (int j = 0; j < kDecVPT; ++j) {
+            if (sv[j] == 0u) continue;  // vertices past the end have no copies
+            const unsigned stid = a.sidx ? a.sidx[v0 + j] : v0 + j;
+            for (unsigned k = 0; k < sv[j]; ++k, ++pos) s_stage[pos] = stid;
+        }
+        __syncthreads();
+        for (unsigned e = tid; e < total; e += kSmallThreads) {
+            if (e < room) q[e] = s_stage[e];
+            else flags |= NRRS_DEV_OVERFLOW;
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < kDecVPT; ++j)
+            for (unsigned k = 0; k < sv[j]; ++k, ++pos) {
+                if (pos < room) q[pos] = a.sidx ? a.sidx[v0 + j] : v0 + j;
+                else flags |= NRRS_DEV_OVERFLOW;
+            }
     }
     if (flags) atomicOr(&a.scr->status, flags);
 }
@@ -612,13 +724,43 @@ cudaError_t launch_decide(const DecideArgs& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_decide_two_pass(const DecideArgs& a, cudaStream_t s) {
+namespace {
+// launch with programmatic stream serialisation (the kernel waits by itself, wait_for_stream), in
+// clusters of `cluster` CTAs
+template <class... A>
+cudaError_t launch_early(void (*k)(A...), unsigned grid, unsigned threads, unsigned cluster,
+                         cudaStream_t s, const A&... args) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(threads);
+    c.stream = s;
+    cudaLaunchAttribute at[2]{};
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = cluster;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    c.attrs = at;
+    c.numAttrs = cluster ? 2 : 1;
+    return cudaLaunchKernelEx(&c, k, args...);
+}
+}  // namespace
+
+int decide_launches(const DecideArgs& a) {
+    return a.segs.n == 1 && a.segs.s[0].count <= 8 * kSmallSpan ? 1 : 2;
+}
+
+cudaError_t launch_decide_context(const DecideArgs& a, cudaStream_t s) {
     if (a.segs.total_tiles == 0) return cudaSuccess;
-    k_decide_count<<<a.segs.total_tiles, kDecThreads, 0, s>>>(a);
-    cudaError_t e = cudaGetLastError();
+    if (decide_launches(a) == 1) {
+        unsigned ctas = 1;
+        while (ctas * kSmallSpan < a.segs.s[0].count) ctas *= 2;
+        return launch_early(k_decide_small, ctas, kSmallThreads, ctas, s, a);
+    }
+    const cudaError_t e =
+        launch_early(k_decide_count, a.segs.total_tiles, kDecThreads, 0u, s, a);
     if (e != cudaSuccess) return e;
-    k_decide_emit<<<a.segs.total_tiles, kDecThreads, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_early(k_decide_emit, a.segs.total_tiles, kDecThreads, 0u, s, a);
 }
 
 cudaError_t launch_sum(const SumArgs& a, cudaStream_t s) {

@@ -112,9 +112,11 @@ extern thread_local int g_last_grid;
 
 // decision + emission (single pass, decoupled look-back)
 cudaError_t launch_decide(const DecideArgs& a, cudaStream_t s);
-// the same decision and queue in two passes without a look-back (count + prefix scan, emission);
-// needs a.split (the caller's array or context scratch of one byte per vertex)
-cudaError_t launch_decide_two_pass(const DecideArgs& a, cudaStream_t s);
+// the same decision and queue without a look-back: one cluster for a single short segment, else two
+// passes (count + prefix scan, emission), which need a.split (the caller's array or context scratch
+// of one byte per vertex); the kernels it launches
+cudaError_t launch_decide_context(const DecideArgs& a, cudaStream_t s);
+int decide_launches(const DecideArgs& a);
 // device-side segment tables of device-resident queue sizes (counts_dev[host_max.n]), in units
 // of kTile (tiles_dev) and kDecChunk (chunks_dev); counts above the host maxima are clamped and
 // flag NRRS_DEV_OVERFLOW in *status

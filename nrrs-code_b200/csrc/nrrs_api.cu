@@ -389,8 +389,8 @@ int run_decide(nrrs_ctx* ctx, const float* rrs, const float* rnd, const uint32_t
     cudaError_t e;
     {
         ProfScope ps(ctx, NRRS_KERNEL_DECIDE, s);
-        e = launch_decide_two_pass(d, s);
-        ++ctx->prof.total_launches;  // the scope counts one of its two kernels
+        e = launch_decide_context(d, s);
+        ctx->prof.total_launches += decide_launches(d) - 1;  // the scope counts one kernel
     }
     if (e != cudaSuccess) {
         cudaMemsetAsync(ctx->scr, 0, offsetof(DecideScratch, epoch), s);
