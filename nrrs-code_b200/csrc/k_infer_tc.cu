@@ -44,6 +44,7 @@ struct PackedNet {
 };
 
 constexpr int cmax(int a, int b) { return a > b ? a : b; }
+constexpr int cmin(int a, int b) { return a < b ? a : b; }
 constexpr int tmem_cols(int w) { return w <= 32 ? 32 : (w <= 64 ? 64 : (w <= 128 ? 128 : 256)); }
 
 // PART: 0 = both networks in one kernel; 1 = StatNet only (writes the RRSNet input tiles);
@@ -573,6 +574,205 @@ __global__ void __launch_bounds__(128 * WGS, (WGS == 2 && WS <= 64 && !TA) ? 3 :
     }
 }
 
+// Short queues: 32 vertices per CTA, so that a queue of a few thousand vertices spreads over all
+// SMs, and every phase is as short as its latencies allow. The four warps gather the same 32
+// vertices' features together (4 levels each: one round of loads where a thread per vertex makes
+// four), then the first warp alone runs the chain on rows 0-31 of the MMA's 128 (the others hold
+// whatever they held; rows do not mix), with warp barriers in place of the warpgroup's. The weights
+// arrive during the gathers. Same arithmetic as k_infer_tc, same bits.
+// A 128-vertex tile costs its SM 128 x 66 gather requests (4.3 us at one per cycle) before its first
+// MMA. 3,071 vertices, 64 x 2: 9.4 us against 18.0 (24 tiles on 12 SMs); bound by the latencies of
+// one round of loads and six MMA layers.
+constexpr int kSmallRows = 32;
+
+template <int WS, int HS, int WR, int HR, bool BF>
+__global__ void __launch_bounds__(128) k_infer_small(const __grid_constant__ InferArgs a) {
+    using S = TcShape<WS, HS, WR, HR, 1, false, 0>;
+    constexpr bool REF = WS == 32;
+    constexpr int KIN = stat_in_of(WS);
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* base = reinterpret_cast<uint8_t*>(
+        (reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~uintptr_t(1023));
+    uint8_t* sW = base;
+    uint8_t* sA = base + S::kAOff;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(base + S::kBarOff);   // weights, mma
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 2);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        tc::mbar_init(&bars[0], 1);
+        tc::mbar_init(&bars[1], 1);
+        tc::fence_mbar_init();
+    }
+    if (warp == 0) {
+        tc::tmem_alloc(tslot, S::kCols);
+        tc::tmem_relinquish();
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    const uint32_t tmem = *tslot;
+    if (tid == 0) {
+        tc::mbar_arrive_expect_tx(&bars[0], S::kWBytes);
+        const uint8_t* src = reinterpret_cast<const uint8_t*>(a.wpack);
+        for (uint32_t off = 0; off < S::kWBytes; off += 32768u) {
+            const uint32_t bytes = S::kWBytes - off < 32768u ? S::kWBytes - off : 32768u;
+            tc::bulk_g2s(sW + off, src + off, bytes, &bars[0]);
+        }
+    }
+    const uint8_t* wS0 = sW;
+    const uint8_t* wSh = wS0 + WS * KIN * 2;
+    const uint8_t* wSo = wSh + (HS - 1) * WS * WS * 2;
+    const uint8_t* wR0 = wSo + 16 * WS * 2;
+    const uint8_t* wRh = wR0 + WR * kRrsIn * 2;
+    const uint8_t* wRo = wRh + (HR - 1) * WR * WR * 2;
+
+    const SegmentTable& ST = seg_table(a.segs);
+    const uint32_t items = ST.total_tiles * (kTile / kSmallRows);
+    const __half2* table = reinterpret_cast<const __half2*>(a.table_h);
+    uint32_t phase = 0;
+    bool ok = true;
+    // the chain's operands are visible to the tensor cores and the warp is together again
+    auto warp_sync_for_mma = [&]() {
+        tc::fence_async_smem();
+        tc::fence_before_sync();
+        __syncwarp();
+    };
+    const uint32_t u = blockIdx.x;   // one item per CTA
+    if (u < items) {
+        const uint32_t t = u / (kTile / kSmallRows), part = u % (kTile / kSmallRows);
+        const int si = find_segment(ST, t);
+        const Segment& sg = ST.s[si];
+        const uint32_t i = sg.offset + (t - sg.tile_start) * kTile + part * kSmallRows + lane;
+        const bool valid = i < sg.offset + sg.count;
+        VertexAux aux{};
+        if (warp == 0 && valid) aux = load_aux(a.v, i);
+        if (valid) {
+            if (warp < (int)(REF ? kRefLevels : kMaxLevels) / 4) {
+                float p[3], f[8];
+                norm_pos(a.enc, a.v.pos, i, p);
+                levels_features_h<4>(table, a.enc, p, 4 * warp, f);
+                store_chunk(sA, lane, warp, KIN, pack8<BF>(f));
+            }
+            if constexpr (REF) {
+                if (warp >= 2) {
+                    float blob[16];
+                    ref_blob_lanes(a.v, i, blob);
+                    store_chunk(sA, lane, warp, KIN, pack8<BF>(warp == 2 ? blob : blob + 8));
+                }
+            } else if (warp == 1) {
+                float sh[16];
+                const size_t i3 = 3 * (size_t)i;
+                sh16(a.v.wi[i3], a.v.wi[i3 + 1], a.v.wi[i3 + 2], sh);
+                store_chunk(sA, lane, 4, KIN, pack8<BF>(sh));
+                store_chunk(sA, lane, 5, KIN, pack8<BF>(sh + 8));
+            } else if (warp == 2) {
+                float misc[16];
+                misc_lanes(a.v, i, misc);
+                store_chunk(sA, lane, 6, KIN, pack8<BF>(misc));
+            } else if (warp == 3) {
+                store_chunk(sA, lane, 7, KIN, make_uint4(0u, 0u, 0u, 0u));
+            }
+        } else if (warp == 0) {
+            zero_row(sA, lane, KIN);
+        }
+        tc::fence_async_smem();
+        __syncthreads();
+        if (warp == 0) {
+            ok = tc::mbar_wait(&bars[0], 0, kSpin);
+            if (ok) {
+                float y[16], r[16], x1[16];
+                ok &= tc_layer<KIN, WS, BF>(sA, wS0, tmem, &bars[1], phase, lane);
+                epilogue_act<WS, BF, REF>(tmem, sA, lane);
+                warp_sync_for_mma();
+#pragma unroll 1
+                for (int h = 1; h < HS; ++h) {
+                    ok &= tc_layer<WS, WS, BF>(sA, wSh + (h - 1) * WS * WS * 2, tmem, &bars[1],
+                                               phase, lane);
+                    epilogue_act<WS, BF, REF>(tmem, sA, lane);
+                    warp_sync_for_mma();
+                }
+                ok &= tc_layer<WS, 16, BF>(sA, wSo, tmem, &bars[1], phase, lane);
+                tc::tmem_ld16(tmem, y);
+                tc::tmem_wait_ld();
+                if (valid) {
+                    if constexpr (REF) glue16_ref_aux(y, aux, x1);
+                    else glue16_aux(a.fp, y, aux, x1);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) x1[k] = 0.f;
+                }
+                store_chunk(sA, lane, 0, 16, pack8<BF>(x1));
+                store_chunk(sA, lane, 1, 16, pack8<BF>(x1 + 8));
+                warp_sync_for_mma();
+                ok &= tc_layer<kRrsIn, WR, BF>(sA, wR0, tmem, &bars[1], phase, lane);
+                epilogue_act<WR, BF, REF>(tmem, sA, lane);
+                warp_sync_for_mma();
+#pragma unroll 1
+                for (int h = 1; h < HR; ++h) {
+                    ok &= tc_layer<WR, WR, BF>(sA, wRh + (h - 1) * WR * WR * 2, tmem, &bars[1],
+                                               phase, lane);
+                    epilogue_act<WR, BF, REF>(tmem, sA, lane);
+                    warp_sync_for_mma();
+                }
+                ok &= tc_layer<WR, 16, BF>(sA, wRo, tmem, &bars[1], phase, lane);
+                tc::tmem_ld16(tmem, r);
+                tc::tmem_wait_ld();
+                tc::fence_before_sync();
+                long long term = 0;
+                if (valid) {
+                    if (a.stats) {
+#pragma unroll
+                        for (int k = 0; k < stat_out_of(WS); ++k)
+                            a.stats[stat_out_of(WS) * (size_t)i + k] = y[k];
+                    }
+                    const float rrs = rrs_factor_aux<REF>(a.fp, y, r[0], aux);
+                    a.rrs[i] = rrs;
+                    if (a.scr || a.ext_acc)
+                        term = fixed_term(a.fp, rrs, a.scr ? &a.scr->status : &g_dummy_status);
+                }
+                if (a.scr || a.ext_acc) {
+                    term = warp_sum_ll(term);
+                    if (lane == 0 && term != 0)
+                        atomicAdd(a.ext_acc ? a.ext_acc : &a.scr->sum_acc[si],
+                                  (unsigned long long)term);
+                }
+            }
+        }
+    } else if (warp == 0) {
+        // a queue shorter than the host's bound: the weights land before the CTA leaves
+        ok = tc::mbar_wait(&bars[0], 0, kSpin);
+    }
+    if (!__all_sync(0xffffffffu, ok) && lane == 0 && a.scr)
+        atomicOr(&a.scr->status, NRRS_DEV_TIMEOUT);
+    tc::fence_before_sync();
+    __syncthreads();
+    if (warp == 0) {
+        tc::fence_after_sync();
+        tc::tmem_dealloc(tmem, S::kCols);
+    }
+}
+
+// CTAs per SM of the short-queue kernel: what shared memory holds, at most 4
+template <int WS, int HS>
+constexpr uint32_t small_ctas() {
+    return cmin(4, (int)(233472u / (TcShape<WS, HS, WS, HS, 1, false, 0>::kSmem + 1024u)));
+}
+
+template <int WS, int HS, int WR, int HR, bool BF>
+cudaError_t launch_small(const InferArgs& a, cudaStream_t s) {
+    using S = TcShape<WS, HS, WR, HR, 1, false, 0>;
+    static_assert(small_ctas<WS, HS>() >= 1 && small_ctas<WS, HS>() * S::kCols <= 512, "one wave");
+    auto kern = k_infer_small<WS, HS, WR, HR, BF>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)S::kSmem);
+    if (e != cudaSuccess) return e;
+    const unsigned grid = a.segs.total_tiles * (kTile / kSmallRows);
+    if (grid == 0) return cudaSuccess;
+    g_last_grid = (int)grid;
+    kern<<<grid, 128, S::kSmem, s>>>(a);
+    return cudaGetLastError();
+}
+
 template <int WS, int HS, int WR, int HR, bool BF, int WGS, bool PRE, int PART, bool TA = false>
 cudaError_t launch_tc(const InferArgs& a, int sm_count, int ctas_per_sm, cudaStream_t s) {
     using S = TcShape<WS, HS, WR, HR, WGS, PRE, PART, TA>;
@@ -719,6 +919,31 @@ cudaError_t launch_infer_tc(const InferArgs& a, int ws, int hs, int wr, int hr, 
                       : launch_tc<32, 3, 32, 3, false, 1, false, 0>(a, sm_count, ctas_per_sm, s);
         return cudaErrorInvalidConfiguration;
     }
+    return cudaErrorInvalidValue;
+}
+
+// One wave of the short-queue kernel: a CTA per 32 vertices, all resident. Measured at the line, per
+// step with the decision (this kernel / k_infer_tc): 64 x 2 networks 16,000 vertices 22 / 32 us,
+// 50,000 vertices (2.6 waves) 37 / 39, 100,000 68 / 54; 128 x 3, whose weights leave one CTA per SM,
+// 3,071 vertices 20 / 33, 8,000 (1.7 waves) 29 / 28; shipped network, 16,000 19 / 23, 30,000 27 / 23.
+bool infer_small_fits(const SegmentTable& segs, int ws, int hs, int sm_count) {
+    const uint32_t per_sm = ws == 128 ? small_ctas<128, 3>()
+                            : ws == 32 ? small_ctas<32, 3>()
+                                       : (hs == 2 ? small_ctas<64, 2>() : small_ctas<64, 3>());
+    return segs.total_tiles * (kTile / kSmallRows) <= (uint32_t)sm_count * per_sm;
+}
+
+cudaError_t launch_infer_small(const InferArgs& a, int ws, int hs, int prec, cudaStream_t s) {
+    const bool bf = prec == NRRS_PREC_BF16;
+    if (ws == 64 && hs == 2)
+        return bf ? launch_small<64, 2, 64, 2, true>(a, s) : launch_small<64, 2, 64, 2, false>(a, s);
+    if (ws == 64 && hs == 3)
+        return bf ? launch_small<64, 3, 64, 3, true>(a, s) : launch_small<64, 3, 64, 3, false>(a, s);
+    if (ws == 128 && hs == 3)
+        return bf ? launch_small<128, 3, 128, 3, true>(a, s)
+                  : launch_small<128, 3, 128, 3, false>(a, s);
+    if (ws == 32 && hs == 3)
+        return bf ? launch_small<32, 3, 32, 3, true>(a, s) : launch_small<32, 3, 32, 3, false>(a, s);
     return cudaErrorInvalidValue;
 }
 

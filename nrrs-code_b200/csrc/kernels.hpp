@@ -137,6 +137,9 @@ int infer_max_ctas(int ws, int hs, int wr, int hr, int prec, int wgs, int split 
 cudaError_t launch_infer_tc(const InferArgs& a, int ws, int hs, int wr, int hr, int prec,
                             int sm_count, int ctas_per_sm, int wgs, int part, bool tmem_act,
                             cudaStream_t s);
+// the short-queue kernel of the same path (any mode's results): which queues it takes, its launch
+bool infer_small_fits(const SegmentTable& segs, int ws, int hs, int sm_count);
+cudaError_t launch_infer_small(const InferArgs& a, int ws, int hs, int prec, cudaStream_t s);
 size_t infer_tc_smem_bytes(int ws, int hs, int wr, int hr);
 // derived weight copies: FP32 transposed and the UMMA-packed FP16/BF16 images
 cudaError_t launch_pack_weights(const float* master_mlp, float* wt, float* wrow, void* wpack,
