@@ -393,16 +393,6 @@ __device__ __forceinline__ unsigned decide_run(const DecideArgs& a, float scale,
     return local;
 }
 
-// waits for the kernels before this one in its stream (and has their writes visible); a kernel
-// launched with programmatic stream serialisation calls it before it touches memory
-__device__ __forceinline__ void wait_for_stream() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-// lets the next kernel of the stream be set up while this one finishes
-__device__ __forceinline__ void let_next_start() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 __global__ void __launch_bounds__(kDecThreads) k_decide_count(const __grid_constant__ DecideArgs a) {
     __shared__ unsigned s_red[kDecThreads / 32];
     __shared__ int s_last;
@@ -724,28 +714,6 @@ cudaError_t launch_decide(const DecideArgs& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-namespace {
-// launch with programmatic stream serialisation (the kernel waits by itself, wait_for_stream), in
-// clusters of `cluster` CTAs
-template <class... A>
-cudaError_t launch_early(void (*k)(A...), unsigned grid, unsigned threads, unsigned cluster,
-                         cudaStream_t s, const A&... args) {
-    cudaLaunchConfig_t c{};
-    c.gridDim = dim3(grid);
-    c.blockDim = dim3(threads);
-    c.stream = s;
-    cudaLaunchAttribute at[2]{};
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = cluster;
-    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
-    c.attrs = at;
-    c.numAttrs = cluster ? 2 : 1;
-    return cudaLaunchKernelEx(&c, k, args...);
-}
-}  // namespace
-
 int decide_launches(const DecideArgs& a) {
     return a.segs.n == 1 && a.segs.s[0].count <= 8 * kSmallSpan ? 1 : 2;
 }
@@ -755,12 +723,12 @@ cudaError_t launch_decide_context(const DecideArgs& a, cudaStream_t s) {
     if (decide_launches(a) == 1) {
         unsigned ctas = 1;
         while (ctas * kSmallSpan < a.segs.s[0].count) ctas *= 2;
-        return launch_early(k_decide_small, ctas, kSmallThreads, ctas, s, a);
+        return launch_early(k_decide_small, ctas, kSmallThreads, 0, ctas, s, a);
     }
     const cudaError_t e =
-        launch_early(k_decide_count, a.segs.total_tiles, kDecThreads, 0u, s, a);
+        launch_early(k_decide_count, a.segs.total_tiles, kDecThreads, 0, 0, s, a);
     if (e != cudaSuccess) return e;
-    return launch_early(k_decide_emit, a.segs.total_tiles, kDecThreads, 0u, s, a);
+    return launch_early(k_decide_emit, a.segs.total_tiles, kDecThreads, 0, 0, s, a);
 }
 
 cudaError_t launch_sum(const SumArgs& a, cudaStream_t s) {

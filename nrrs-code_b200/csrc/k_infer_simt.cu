@@ -61,6 +61,7 @@ __global__ void __launch_bounds__(FpShape<WS>::kThr, WS == 128 ? 4 : 8)
     extern __shared__ float4 smem4[];
     float* act = reinterpret_cast<float*>(smem4);
     float* wch = act + S::kActFloats;
+    wait_for_stream();
     const int tid = threadIdx.x;
     const int m = tid & (kTM - 1);
     const bool lead = tid < kTM;               // the thread that owns vertex column m
@@ -173,8 +174,7 @@ cudaError_t launch_cfg(const InferArgs& a, int sm_count, int ctas_per_sm, cudaSt
     if (grid > items) grid = items;
     if (grid == 0) return cudaSuccess;
     g_last_grid = (int)grid;
-    kern<<<grid, S::kThr, S::kSmem, s>>>(a);
-    return cudaGetLastError();
+    return launch_early(kern, grid, S::kThr, S::kSmem, 0, s, a);
 }
 
 }  // namespace

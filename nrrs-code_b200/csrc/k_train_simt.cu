@@ -184,6 +184,7 @@ __global__ void __launch_bounds__(TrShape<WS>::kThr, WS == 128 ? 4 : 8)
     float* tile = reinterpret_cast<float*>(smem4);
     float* wch = tile + S::kRows * kTM;
     __shared__ double red[S::kThr / 32];
+    wait_for_stream();
     const int tid = threadIdx.x;
     const int m = tid & (kTM - 1);
     const bool lead = tid < kTM;
@@ -367,6 +368,7 @@ __global__ void __launch_bounds__(TrShape<WR>::kThr, WR == 128 ? 4 : 8)
     float* tile = reinterpret_cast<float*>(smem4);
     float* wch = tile + S::kRows * kTM;
     __shared__ double s_tot[4], s_red[4][S::kThr / 4];
+    wait_for_stream();
     const int tid = threadIdx.x;
     const int m = tid & (kTM - 1);
     const bool lead = tid < kTM;
@@ -668,6 +670,7 @@ constexpr WShape kWShapes[] = {{64, 64}, {32, 32}, {64, 16}, {32, 16}, {8, 64}, 
 __global__ void __launch_bounds__(kWThr, 2) k_wgrad(const __grid_constant__ WGradArgs a) {
     extern __shared__ float4 smem4[];
     float* sm = reinterpret_cast<float*>(smem4);
+    wait_for_stream();
     const WJob& j = a.job[blockIdx.y];
     const uint32_t i0 = blockIdx.x * a.chunk;
     const uint32_t i1 = min(a.n, i0 + a.chunk);
@@ -724,6 +727,7 @@ __global__ void __launch_bounds__(32 * kRedSlices) k_wreduce(const float* partia
                                                              uint32_t stride, uint32_t count,
                                                              float* grad, float scale) {
     __shared__ float red[kRedSlices][32];
+    wait_for_stream();
     const uint32_t lane = threadIdx.x & 31u, sl = threadIdx.x >> 5;
     const uint32_t e = blockIdx.x * 32u + lane;
     const uint32_t per = (chunks + kRedSlices - 1) / kRedSlices;
@@ -830,6 +834,7 @@ struct EmaArgs {
 // the moving average after an Adam step: e = d e + (1 - d) w, pi = e / (1 - d^t), each product
 // and the sum rounded separately (no contraction), so a float32 restatement gives the same bits
 __global__ void k_ema(const __grid_constant__ EmaArgs a) {
+    wait_for_stream();
     for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < a.count;
          k += (uint64_t)gridDim.x * blockDim.x) {
         const float e = __fadd_rn(__fmul_rn(a.d, a.e[k]), __fmul_rn(a.omd, a.p[k]));
@@ -858,15 +863,11 @@ cudaError_t launch_train(nrrs_ctx* ctx, TrainArgs& a, cudaStream_t s, AfterStat 
     a.part_n = grid;
     {
         ProfScope ps(ctx, NRRS_KERNEL_TRAIN_STAT, s);
-        ks<<<grid, kThr, smem, s>>>(a);
+        e = launch_early(ks, grid, kThr, smem, 0, s, a);
     }
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = after_stat()) != cudaSuccess) return e;
-    {
-        ProfScope ps(ctx, NRRS_KERNEL_TRAIN_RRS, s);
-        kr<<<grid, kThr, smem, s>>>(a);
-    }
-    return cudaGetLastError();
+    if (e != cudaSuccess || (e = after_stat()) != cudaSuccess) return e;
+    ProfScope ps(ctx, NRRS_KERNEL_TRAIN_RRS, s);
+    return launch_early(kr, grid, kThr, smem, 0, s, a);
 }
 
 struct Layout {
@@ -896,12 +897,12 @@ uint32_t ld_of(uint32_t n) { return (n + 127) / 128 * 128; }
 
 cudaError_t launch_wreduce(const float* partial, uint32_t chunks, uint32_t stride, uint32_t count,
                            float* grad, float scale, cudaStream_t s) {
-    k_wreduce<<<(count + 31) / 32, 32 * kRedSlices, 0, s>>>(partial, chunks, stride, count, grad,
-                                                            scale);
-    return cudaGetLastError();
+    return launch_early(k_wreduce, (count + 31) / 32, 32u * kRedSlices, 0, 0, s, partial, chunks,
+                        stride, count, grad, scale);
 }
 
-// Adam over the trained parameters: table + StatNet (+ RRSNet at step 3); refreshes the FP16 table
+// Adam over the trained parameters: table + StatNet (+ RRSNet at step 3); refreshes the FP16 tables
+// (the caller rebuilds the other derived images)
 cudaError_t launch_adam_step(nrrs_ctx* ctx, bool train_rrs, cudaStream_t s, float scale) {
     const nrrs_config& c = ctx->cfg;
     ctx->adam_t += 1;
@@ -928,11 +929,7 @@ cudaError_t launch_adam_step(nrrs_ctx* ctx, bool train_rrs, cudaStream_t s, floa
         ProfScope ps(ctx, NRRS_KERNEL_ADAM, s);
         k_adam<<<(unsigned)ctx->sm_count * 8, 256, 0, s>>>(ad);
     }
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess && ctx->cells) {
-        ProfScope ps(ctx, NRRS_KERNEL_CELL_IMAGE, s);
-        e = launch_cell_image(ctx->table_h, half_enc(ctx), ctx->cells, ctx->n_cells, ctx->sm_count, s);
-    }
+    const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || !ctx->ema) return e;
     // the moving average of every parameter and the inference table derived from it
     ctx->ema_t += 1;
@@ -948,13 +945,8 @@ cudaError_t launch_adam_step(nrrs_ctx* ctx, bool train_rrs, cudaStream_t s, floa
     ea.inv = (float)(1.0 / (1.0 - std::pow((double)c.ema_decay, (double)ctx->ema_t)));
     {
         ProfScope ps(ctx, NRRS_KERNEL_ADAM, s);
-        k_ema<<<(unsigned)ctx->sm_count * 8, 256, 0, s>>>(ea);
+        return launch_early(k_ema, (unsigned)ctx->sm_count * 8, 256, 0, 0, s, ea);
     }
-    e = cudaGetLastError();
-    if (e != cudaSuccess || !ctx->cells_inf) return e;
-    ProfScope ps(ctx, NRRS_KERNEL_CELL_IMAGE, s);
-    return launch_cell_image(ctx->table_h_inf, half_enc(ctx), ctx->cells_inf, ctx->n_cells,
-                             ctx->sm_count, s);
 }
 
 bool train_tc_supported(const nrrs_config& c);
@@ -1112,8 +1104,7 @@ int train_step_impl(nrrs_ctx* ctx, const VertexPtrs& v, const float* target, uin
     e = cudaFuncSetAttribute(k_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWSmem);
     if (e == cudaSuccess) {
         ProfScope ps(ctx, NRRS_KERNEL_TRAIN_WGRAD, s);
-        k_wgrad<<<dim3((unsigned)chunks, (unsigned)nj), kWThr, kWSmem, s>>>(w);
-        e = cudaGetLastError();
+        e = launch_early(k_wgrad, dim3((unsigned)chunks, (unsigned)nj), kWThr, kWSmem, 0, s, w);
     }
     if (e == cudaSuccess) {
         // the first `off` entries have partials; gradients of untrained layers stay zero

@@ -56,7 +56,7 @@ struct TcTrainArgs {
     float* dxs;             // when set: per-sample hash-lane gradients [n][32] out, no scatter here
     double* part;           // [part_rows][4]: loss_S, V, C, R per CTA
     uint32_t part_rows;
-    uint32_t part_used;     // rows the StatNet and RRSNet-forward grids write
+    uint32_t part_stat, part_rrs;   // rows the StatNet (column 0) and RRSNet-forward grids write
     double* loss_out;
     LossWeights lw;         // per-sample loss weights (inactive: plain means)
     unsigned* status;       // the context's NRRS_DEV_* word: wait timeouts are reported there
@@ -166,6 +166,7 @@ __global__ void __launch_bounds__(128 * WGS, 1) k_ttc_stat(const __grid_constant
     __shared__ int s_abort[WGS];
     __shared__ double red[4 * WGS];
 
+    wait_for_stream();
     if (threadIdx.x == 0) {
         for (int k = 0; k < (int)S::kNumBars; ++k) tc::mbar_init(&bars[k], 1);
         tc::fence_mbar_init();
@@ -471,6 +472,7 @@ __global__ void __launch_bounds__(128 * WGS, 1) k_ttc_rrs(const __grid_constant_
     __shared__ double red[4 * WGS];
     __shared__ double s_tot[4];
 
+    wait_for_stream();
     if (threadIdx.x == 0) {
         for (int k = 0; k < (int)S::kNumBars; ++k) tc::mbar_init(&bars[k], 1);
         tc::fence_mbar_init();
@@ -480,8 +482,8 @@ __global__ void __launch_bounds__(128 * WGS, 1) k_ttc_rrs(const __grid_constant_
         // batch sums of the loss partials (rows written by the StatNet and forward launches),
         // in a fixed order, so every CTA holds the same V and C
         double t0 = 0.0, t1 = 0.0, t2 = 0.0, t3 = 0.0;
-        for (uint32_t b = threadIdx.x; b < a.part_used; b += blockDim.x) {
-            t0 += a.part[4 * b + 0];
+        for (uint32_t b = threadIdx.x; b < a.part_stat; b += blockDim.x) t0 += a.part[4 * b + 0];
+        for (uint32_t b = threadIdx.x; b < a.part_rrs; b += blockDim.x) {
             t1 += a.part[4 * b + 1];
             t2 += a.part[4 * b + 2];
             t3 += a.part[4 * b + 3];
@@ -696,6 +698,7 @@ __global__ void __launch_bounds__(128, 1) k_wgrad_tc(const __grid_constant__ TcW
     const uint32_t s1 = min(a.n, s0 + a.chunk);
     const uint32_t stages = (s1 - s0 + 63) / 64;
 
+    wait_for_stream();
     if (tid == 0) {
         for (int k = 0; k < 5; ++k) tc::mbar_init(&bars[k], 1);
         tc::fence_mbar_init();
@@ -758,6 +761,10 @@ __global__ void __launch_bounds__(128, 1) k_wgrad_tc(const __grid_constant__ TcW
         if (j.Fa == 64) wgrad_epilogue<64>(trow, j, out, m);
         else if (j.Fa == 16) wgrad_epilogue<16>(trow, j, out, m);
         else wgrad_epilogue<128>(trow, j, out, m);
+    } else if ((uint32_t)tid < j.Mv) {
+        // a wait that ran out: no gradient from this chunk
+        float* out = a.partial + (size_t)c * a.total + j.out + (size_t)tid * j.ldw;
+        for (uint32_t k = 0; k < j.Nv; ++k) out[k] = 0.f;
     }
     if (tid == 0 && (s_fail || !done)) atomicOr(a.status, NRRS_DEV_TIMEOUT);
     tc::fence_before_sync();
@@ -824,25 +831,18 @@ cudaError_t launch_ttc(nrrs_ctx* ctx, TcTrainArgs& a, cudaStream_t s, bool train
     };
     const uint32_t gs = grid_of((const void*)ks, SS::kSmem);
     const uint32_t g = grid_of((const void*)kr0, RS::kSmem);
-    a.part_used = gs > g ? gs : g;
-    if (a.part_used > a.part_rows) return cudaErrorInvalidConfiguration;
+    a.part_stat = gs;
+    a.part_rrs = train_rrs ? g : 0;   // without the RRSNet only the StatNet sum is present
+    if (gs > a.part_rows || g > a.part_rows) return cudaErrorInvalidConfiguration;
     {
         ProfScope ps(ctx, NRRS_KERNEL_TRAIN_STAT, s);
-        ks<<<gs, kThreads, SS::kSmem, s>>>(a);
+        e = launch_early(ks, gs, kThreads, SS::kSmem, 0, s, a);
     }
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = after_stat()) != cudaSuccess) return e;
-    if (train_rrs) {
-        ProfScope ps(ctx, NRRS_KERNEL_TRAIN_RRS, s);
-        kr0<<<g, kThreads, RS::kSmem, s>>>(a);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        kr1<<<g, kThreads, RS::kSmem, s>>>(a);
-    } else {
-        // losses without the RRSNet: only the StatNet sum is present
-        ProfScope ps(ctx, NRRS_KERNEL_TRAIN_RRS, s);
-        kr1<<<1, kThreads, RS::kSmem, s>>>(a);
-    }
-    return cudaGetLastError();
+    if (e != cudaSuccess || (e = after_stat()) != cudaSuccess) return e;
+    ProfScope ps(ctx, NRRS_KERNEL_TRAIN_RRS, s);
+    if (train_rrs) e = launch_early(kr0, g, kThreads, RS::kSmem, 0, s, a);
+    if (e != cudaSuccess) return e;
+    return launch_early(kr1, train_rrs ? g : 1u, kThreads, RS::kSmem, 0, s, a);
 }
 
 }  // namespace
@@ -941,12 +941,13 @@ int train_step_tc(nrrs_ctx* ctx, const VertexPtrs& v, const float* target, uint3
         (reinterpret_cast<uintptr_t>(partial + chunks_max * mlp) + 15u) & ~uintptr_t(15));
     const bool split = ctx->train_split != 0;
     // the split step zeroes the table gradient level group by level group right before that
-    // group's scatter (below); here only what the other kernels accumulate into
-    const uint64_t zero_from = split ? ctx->n_table : 0;
-    cudaError_t e = cudaMemsetAsync(ctx->grads + zero_from, 0,
-                                    sizeof(float) * (ctx->n_params - zero_from), s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(part, 0, sizeof(double) * 4 * part_rows, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(partial, 0, sizeof(float) * chunks * mlp, s);
+    // group's scatter (below), and the reduction writes the trained layers' gradients; here only
+    // what is left
+    cudaError_t e = cudaSuccess;
+    if (!split) e = cudaMemsetAsync(ctx->grads, 0, sizeof(float) * ctx->n_table, s);
+    if (e == cudaSuccess && !train_rrs)
+        e = cudaMemsetAsync(ctx->grads + ctx->n_table + ctx->n_stat, 0,
+                            sizeof(float) * ctx->n_rrs, s);
     if (e != cudaSuccess) {
         ctx->last_error = std::string("train memset: ") + cudaGetErrorString(e);
         return NRRS_ERR_CUDA;
@@ -1073,13 +1074,12 @@ int train_step_tc(nrrs_ctx* ctx, const VertexPtrs& v, const float* target, uint3
     e = cudaFuncSetAttribute(k_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsm);
     if (e == cudaSuccess) {
         ProfScope ps(ctx, NRRS_KERNEL_TRAIN_WGRAD, s);
-        k_wgrad_tc<<<dim3((unsigned)chunks, (unsigned)nj), 128, wsm, s>>>(w);
-        e = cudaGetLastError();
+        e = launch_early(k_wgrad_tc, dim3((unsigned)chunks, (unsigned)nj), 128, wsm, 0, s, w);
     }
     if (e == cudaSuccess) {
         ProfScope ps(ctx, NRRS_KERNEL_TRAIN_REDUCE, s);
-        e = launch_wreduce(partial, (uint32_t)chunks, (uint32_t)mlp, (uint32_t)mlp,
-                           ctx->grads + ctx->n_table,
+        e = launch_wreduce(partial, (uint32_t)chunks, (uint32_t)mlp,
+                           (uint32_t)(train_rrs ? mlp : ctx->n_stat), ctx->grads + ctx->n_table,
                            1.0f / (float)n, s);
     }
     join();  // the table gradient is complete on s from here

@@ -141,19 +141,63 @@ cudaError_t launch_infer_tc(const InferArgs& a, int ws, int hs, int wr, int hr, 
 bool infer_small_fits(const SegmentTable& segs, int ws, int hs, int sm_count);
 cudaError_t launch_infer_small(const InferArgs& a, int ws, int hs, int prec, cudaStream_t s);
 size_t infer_tc_smem_bytes(int ws, int hs, int wr, int hr);
-// derived weight copies: FP32 transposed and the UMMA-packed FP16/BF16 images
-cudaError_t launch_pack_weights(const float* master_mlp, float* wt, float* wrow, void* wpack,
-                                int ws, int hs, int wr, int hr, int prec, cudaStream_t s);
 size_t packed_weight_bytes(int ws, int hs, int wr, int hr);
 size_t transposed_weight_floats(int ws, int hs, int wr, int hr);
-// BF16 training image: forward layers + transposed layers for input gradients
-cudaError_t launch_pack_train(const float* master_mlp, void* out, int ws, int hs, int wr, int hr,
-                              cudaStream_t s);
 size_t train_pack_bytes(int ws, int hs, int wr, int hr);
 // FP32 table -> FP16 copy
 cudaError_t launch_table_to_half(const float* t, __half* h, size_t n, cudaStream_t s);
-// the cell image of the dense levels (EncodeParams::cells) from the FP16 table
-cudaError_t launch_cell_image(const __half* table_h, const EncodeParams& e, uint4* cells,
-                              uint32_t n_cells, int sm_count, cudaStream_t s);
+// One launch for everything derived from the weights after an update: the MLP images (FP32
+// transposed and row-major copies, the UMMA inference and training images; a null pointer skips
+// one) of up to two parameter vectors, and the cell images (EncodeParams::cells) of up to two FP16
+// tables in the layout of `enc`.
+struct PackArgs {
+    const float* master;   // the MLP part of a parameter vector
+    float* wt;             // [in][out4] per layer
+    float* wrow;           // 16-byte aligned row-major copy (backward passes)
+    void* wpack;           // FP16/BF16 UMMA image (inference)
+    uint16_t* tpack;       // training image: forward layers, FP16 StatNet / BF16 RRSNet
+    int ws, hs, wr, hr, prec;
+};
+struct DeriveArgs {
+    PackArgs pack[2];
+    int n_pack, n_cell;
+    EncodeParams enc;
+    const __half* table_h[2];
+    uint4* cells[2];
+    uint32_t cell_rows;    // (y, z) rows of the dense levels
+};
+cudaError_t launch_derive(const DeriveArgs& a, int sm_count, cudaStream_t s);
+
+// ---- programmatic stream serialisation: a kernel launched by launch_early is set up while the
+// one before it in the stream finishes; it calls wait_for_stream() before it touches memory
+// (2 to 3 us between the kernels of a step become about 1). `cluster` CTAs per cluster, 0 = none.
+template <class... A>
+cudaError_t launch_early(void (*k)(A...), dim3 grid, unsigned threads, size_t smem, unsigned cluster,
+                         cudaStream_t s, const A&... args) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute at[2]{};
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = cluster;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    c.attrs = at;
+    c.numAttrs = cluster ? 2 : 1;
+    const cudaError_t e = cudaLaunchKernelEx(&c, k, args...);
+    if (e != cudaSuccess) cudaGetLastError();   // reported here, not by a later call
+    return e;
+}
+// waits for the kernels before this one in its stream and has their writes visible
+__device__ __forceinline__ void wait_for_stream() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// lets the next kernel of the stream be set up while this one finishes
+__device__ __forceinline__ void let_next_start() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 }  // namespace nrrs

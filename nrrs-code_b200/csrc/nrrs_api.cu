@@ -180,54 +180,46 @@ int ema_restart(nrrs_ctx* ctx, cudaStream_t s) {
 // FP32 MLP weights, the tensor-core training image, the FP16 table and its cell image); from the
 // inference weights (params_inf with a moving average, else params) the inference images (the
 // UMMA weight image, and with a moving average its own transposed weights, FP16 table and cell
-// image). table = false skips the tables (the Adam and moving-average passes wrote them).
+// image). table = false: the Adam and moving-average passes have written the FP16 tables.
 int refresh_derived(nrrs_ctx* ctx, cudaStream_t s, bool table = true) {
     const nrrs_config& c = ctx->cfg;
     const bool ema = ctx->ema != nullptr;
-    cudaError_t e;
-    {
-        ProfScope ps(ctx, NRRS_KERNEL_PACK, s);
-        e = launch_pack_weights(ctx->params + ctx->n_table, ctx->wt, ctx->wrow,
-                                ema ? nullptr : ctx->wpack, c.statnet_width, c.statnet_hidden,
-                                c.rrsnet_width, c.rrsnet_hidden, c.precision, s);
-    }
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "pack weights");
-    if (ema) {
-        ProfScope ps(ctx, NRRS_KERNEL_PACK, s);
-        e = launch_pack_weights(ctx->params_inf + ctx->n_table, ctx->wt_inf, nullptr, ctx->wpack,
-                                c.statnet_width, c.statnet_hidden, c.rrsnet_width,
-                                c.rrsnet_hidden, c.precision, s);
-        if (e != cudaSuccess) return cuda_fail(ctx, e, "pack inference weights");
-    }
-    if (ctx->tpack) {
-        ProfScope ps(ctx, NRRS_KERNEL_PACK, s);
-        e = launch_pack_train(ctx->params + ctx->n_table, ctx->tpack, c.statnet_width,
-                              c.statnet_hidden, c.rrsnet_width, c.rrsnet_hidden, s);
-        if (e != cudaSuccess) return cuda_fail(ctx, e, "pack training weights");
-    }
+    cudaError_t e = cudaSuccess;
     if (ctx->table_h && table) {
         ProfScope ps(ctx, NRRS_KERNEL_TABLE_HALF, s);
         e = launch_table_to_half(ctx->params, ctx->table_h + 2 * ctx->shift_h, ctx->n_table, s);
-        if (e != cudaSuccess) return cuda_fail(ctx, e, "table to half");
+        if (e == cudaSuccess && ema) {
+            ++ctx->prof.total_launches;
+            e = launch_table_to_half(ctx->params_inf, ctx->table_h_inf + 2 * ctx->shift_h,
+                                     ctx->n_table, s);
+        }
     }
-    if (ctx->cells && table) {
-        ProfScope ps(ctx, NRRS_KERNEL_CELL_IMAGE, s);
-        e = launch_cell_image(ctx->table_h, half_enc(ctx), ctx->cells, ctx->n_cells, ctx->sm_count, s);
-        if (e != cudaSuccess) return cuda_fail(ctx, e, "cell image");
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "table to half");
+    DeriveArgs d{};
+    d.pack[d.n_pack++] = PackArgs{ctx->params + ctx->n_table, ctx->wt, ctx->wrow,
+                                  ema ? nullptr : ctx->wpack,
+                                  reinterpret_cast<uint16_t*>(ctx->tpack), c.statnet_width,
+                                  c.statnet_hidden, c.rrsnet_width, c.rrsnet_hidden, c.precision};
+    if (ema)
+        d.pack[d.n_pack++] = PackArgs{ctx->params_inf + ctx->n_table, ctx->wt_inf, nullptr,
+                                      ctx->wpack, nullptr, c.statnet_width, c.statnet_hidden,
+                                      c.rrsnet_width, c.rrsnet_hidden, c.precision};
+    if (ctx->cells) {
+        d.enc = half_enc(ctx);
+        for (uint32_t l = 0; l < d.enc.n_levels; ++l)
+            if (d.enc.lv[l].dense) d.cell_rows += d.enc.lv[l].res * d.enc.lv[l].res;
+        d.table_h[d.n_cell] = ctx->table_h;
+        d.cells[d.n_cell++] = ctx->cells;
+        if (ctx->cells_inf) {
+            d.table_h[d.n_cell] = ctx->table_h_inf;
+            d.cells[d.n_cell++] = ctx->cells_inf;
+        }
     }
-    if (ema && ctx->table_h_inf && table) {
-        ProfScope ps(ctx, NRRS_KERNEL_TABLE_HALF, s);
-        e = launch_table_to_half(ctx->params_inf, ctx->table_h_inf + 2 * ctx->shift_h,
-                                 ctx->n_table, s);
-        if (e != cudaSuccess) return cuda_fail(ctx, e, "inference table to half");
+    {
+        ProfScope ps(ctx, ctx->cells ? NRRS_KERNEL_CELL_IMAGE : NRRS_KERNEL_PACK, s);
+        e = launch_derive(d, ctx->sm_count, s);
     }
-    if (ema && ctx->cells_inf && table) {
-        ProfScope ps(ctx, NRRS_KERNEL_CELL_IMAGE, s);
-        e = launch_cell_image(ctx->table_h_inf, half_enc(ctx), ctx->cells_inf, ctx->n_cells,
-                              ctx->sm_count, s);
-        if (e != cudaSuccess) return cuda_fail(ctx, e, "inference cell image");
-    }
-    return NRRS_OK;
+    return e == cudaSuccess ? NRRS_OK : cuda_fail(ctx, e, "derived images");
 }
 
 int run_infer(nrrs_ctx* ctx, const nrrs_vertex_soa* v, const SegmentTable& segs,
