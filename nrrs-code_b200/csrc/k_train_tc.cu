@@ -387,8 +387,11 @@ __global__ void __launch_bounds__(128 * WGS, 1) k_ttc_stat(const __grid_constant
 // 2^T x 8 bytes), which stays in L2, instead of the whole table. dxs: the per-sample hash-lane
 // gradients that k_ttc_stat wrote, [16][n] float pairs; the 1/n of the batch mean is applied
 // here. Levels [level_begin, level_end) of the launch.
-// FP32 table-gradient bytes per scatter launch of the split step (a fraction of L2)
-constexpr uint64_t kScatterGroupBytes = 40ull << 20;
+// FP32 table-gradient bytes per scatter launch (a fraction of L2): 20 MB beside the mixed step's
+// kernels (64 x 2, 2^19 entries, 262,144 samples: 472 us a step, 477 with 40 MB, 493 with 72, 468
+// with 10; at 2^22 entries a level is 34 MB anyway), 40 MB beside the FP32 step's, which leave few
+// SM slots to start launches in (1,017 us; 1,030 with 20 MB, 1,055 with 10, 1,022 with 72)
+constexpr uint64_t kScatterGroupTc = 20ull << 20, kScatterGroupFp32 = 40ull << 20;
 
 struct ScatterLvArgs {
     EncodeParams enc;
@@ -867,7 +870,7 @@ size_t train_tc_scratch_bytes(const nrrs_config& c, uint32_t n, int sm_count) {
 
 cudaError_t launch_scatter_table(nrrs_ctx* ctx, const float* pos, uint32_t n, const LaneGrads& g,
                                  cudaStream_t s) {
-    // Level groups of at most kScatterGroupBytes of FP32 gradient, each zeroed right before its
+    // Level groups of at most group_bytes of FP32 gradient, each zeroed right before its
     // scatter: the zeroing writes whole sectors into L2, so the reductions that follow hit
     // there. Zeroed at the start of the step, the slices were evicted by the kernels in between,
     // and every first reduction into a sector read its zeros back from HBM as a random 32-byte
@@ -882,6 +885,7 @@ cudaError_t launch_scatter_table(nrrs_ctx* ctx, const float* pos, uint32_t n, co
     const uint32_t g_max =
         (uint32_t)(ctx->sm_count * resident_ctas((const void*)k_scatter_levels, 128, 0, 16));
     const int nl = ctx->cfg.n_levels;
+    const uint64_t group_bytes = train_tc_supported(ctx->cfg) ? kScatterGroupTc : kScatterGroupFp32;
     auto level_rows = [&](int l) -> uint64_t {
         const LevelDev& lv = ctx->enc.lv[l];
         const uint64_t r = (uint64_t)lv.res + 1;
@@ -893,7 +897,7 @@ cudaError_t launch_scatter_table(nrrs_ctx* ctx, const float* pos, uint32_t n, co
         uint64_t row1 = row0 + level_rows(l0);
         int l1 = l0 + 1;
         while (l1 < nl &&
-               (ctx->enc.lv[l1].offset + level_rows(l1) - row0) * 8u <= kScatterGroupBytes) {
+               (ctx->enc.lv[l1].offset + level_rows(l1) - row0) * 8u <= group_bytes) {
             row1 = ctx->enc.lv[l1].offset + level_rows(l1);
             ++l1;
         }
