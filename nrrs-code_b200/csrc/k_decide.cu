@@ -585,6 +585,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_decide_small(const __grid_con
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const unsigned rank = blockIdx.x;
     unsigned flags = 0;
+    let_next_start();
     wait_for_stream();
     const SegmentTable& S = seg_table(a.segs);
     const Segment& sg = S.s[0];

@@ -27,6 +27,7 @@ namespace {
 
 template <bool BF>
 __global__ void __launch_bounds__(kTile) k_encode_levels(const __grid_constant__ EncodeLvArgs a) {
+    wait_for_stream();
     // work items are (level group, tile) over the tiles the host sized the launch for; with
     // device-resident sizes the tiles past the actual total are skipped
     const uint32_t tiles = a.segs.total_tiles;
@@ -60,6 +61,7 @@ __global__ void __launch_bounds__(kTile) k_encode_levels(const __grid_constant__
 // (64 x 2 networks, 262,144 samples: 89 us for the
 // encoding, 330 us inside the training kernel).
 __global__ void __launch_bounds__(kTile) k_encode_f32(const __grid_constant__ EncodeF32Args a) {
+    wait_for_stream();
     const uint32_t tiles = a.tile_end - a.tile_begin;
     const uint32_t items = a.enc.n_levels / 4 * tiles;
     const SegmentTable& S = seg_table(a.segs);
@@ -94,8 +96,7 @@ cudaError_t launch_encode_f32(const EncodeF32Args& a, int sm_count, cudaStream_t
     if (items == 0) return cudaSuccess;
     const uint32_t most =
         (uint32_t)(sm_count * resident_ctas((const void*)k_encode_f32, kTile, 0, 16));
-    k_encode_f32<<<items < most ? items : most, kTile, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_early(k_encode_f32, items < most ? items : most, kTile, 0, 0, s, a);
 }
 
 cudaError_t launch_encode_levels(const EncodeLvArgs& a, bool bf, int sm_count, cudaStream_t s) {
@@ -105,8 +106,7 @@ cudaError_t launch_encode_levels(const EncodeLvArgs& a, bool bf, int sm_count, c
     const int per_sm = resident_ctas((const void*)k, kTile, 0, 16);
     uint32_t grid = (uint32_t)(sm_count * per_sm);
     if (grid > items) grid = items;
-    k<<<grid, kTile, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_early(k, grid, kTile, 0, 0, s, a);
 }
 
 }  // namespace nrrs

@@ -317,6 +317,7 @@ __global__ void __launch_bounds__(128 * WGS, (WGS == 2 && WS <= 64 && !TA) ? 3 :
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = *tslot + (uint32_t)wg * S::kColsWg;
+    wait_for_stream();   // the set-up above touches this CTA's memory only
     if (tid == 0) {
         tc::mbar_arrive_expect_tx(&bars[0], S::kWBytes);
         const uint8_t* src = reinterpret_cast<const uint8_t*>(a.wpack) + S::kWSrcOff;
@@ -611,6 +612,8 @@ __global__ void __launch_bounds__(128) k_infer_small(const __grid_constant__ Inf
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = *tslot;
+    let_next_start();
+    wait_for_stream();   // the set-up above touches this CTA's memory only
     if (tid == 0) {
         tc::mbar_arrive_expect_tx(&bars[0], S::kWBytes);
         const uint8_t* src = reinterpret_cast<const uint8_t*>(a.wpack);
@@ -769,8 +772,7 @@ cudaError_t launch_small(const InferArgs& a, cudaStream_t s) {
     const unsigned grid = a.segs.total_tiles * (kTile / kSmallRows);
     if (grid == 0) return cudaSuccess;
     g_last_grid = (int)grid;
-    kern<<<grid, 128, S::kSmem, s>>>(a);
-    return cudaGetLastError();
+    return launch_early(kern, grid, 128, S::kSmem, 0, s, a);
 }
 
 template <int WS, int HS, int WR, int HR, bool BF, int WGS, bool PRE, int PART, bool TA = false>
@@ -789,8 +791,7 @@ cudaError_t launch_tc(const InferArgs& a, int sm_count, int ctas_per_sm, cudaStr
     if (grid > ctas_needed) grid = ctas_needed;
     if (grid == 0) return cudaSuccess;
     g_last_grid = (int)grid;
-    kern<<<grid, 128 * WGS, S::kSmem, s>>>(a);
-    return cudaGetLastError();
+    return launch_early(kern, grid, 128 * WGS, S::kSmem, 0, s, a);
 }
 
 // part: 0 both networks (fused or split-1), 1 StatNet only, 2 RRSNet only (split-2); tmem_act:

@@ -24,6 +24,7 @@
 //     loaded before any is stored.
 #include <cmath>
 
+#include "launch_early.cuh"
 #include "records.hpp"
 #include "fixed_point.cuh"
 #include "tc_ptx.cuh"
@@ -216,6 +217,7 @@ __device__ __forceinline__ void copy_in(T* dst, const T* __restrict__ src, unsig
 __global__ void __launch_bounds__(kRecThreads) k_record_count(const __grid_constant__ RecordArgs a) {
     __shared__ unsigned s_part[kRecThreads / 32];
     __shared__ unsigned s_last;
+    wait_for_stream();
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const NodeView& nb = a.nb;
     const unsigned c = blockIdx.x, v0 = c * kRecChunk;
@@ -292,6 +294,7 @@ k_record_nodes(const __grid_constant__ RecordArgs a) {
     RecordStage& S = *reinterpret_cast<RecordStage*>(smem_raw);
     __shared__ unsigned s_cnt[kWrPasses * (kWrThreads / 32)];
     __shared__ float s_stage[kWrThreads / 32][96];
+    wait_for_stream();
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const NodeView& nb = a.nb;
     const unsigned c = blockIdx.x, v0 = c * kRecChunk;
@@ -418,6 +421,7 @@ k_record_nodes(const __grid_constant__ RecordArgs a) {
 // ---- recordRadiance for a queue of contributions -------------------------------------------
 __global__ void __launch_bounds__(256) k_record_radiance(const __grid_constant__ RadianceArgs a) {
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+    wait_for_stream();
     if (i >= a.n) return;
     const NodeView& nb = a.nb;
     const int node = a.node[i];
@@ -621,6 +625,7 @@ __global__ void __launch_bounds__(kRecThreads, 5) k_generate(const __grid_consta
     __shared__ LookbackSmem s_lb;
     __shared__ float s_L[kRecPasses][3][kRecThreads];
     __shared__ float s_stage[kRecThreads / 32][96];
+    wait_for_stream();
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const NodeView& nb = a.nb;
     if (tid == 0) s_epoch = *(volatile unsigned*)&nb.hdr[kHdrEpoch];
@@ -781,6 +786,7 @@ __global__ void __launch_bounds__(kRecThreads, 5) k_generate(const __grid_consta
 
 // ---- 1 / samples of the sample's pixel -------------------------------------------------------
 __global__ void __launch_bounds__(256) k_sample_weights(const __grid_constant__ WeightArgs a) {
+    wait_for_stream();
     const unsigned n = min(a.max_n, *a.size_dev);
     for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
         const unsigned px = a.pixel[t];
@@ -808,16 +814,15 @@ cudaError_t launch_record_nodes(const RecordArgs& a, cudaStream_t s) {
         if (e != cudaSuccess) return e;
         attr_set = true;
     }
-    k_record_count<<<a.chunks, kRecThreads, 0, s>>>(a);
-    if (bulk) k_record_nodes<true><<<a.chunks, kWrThreads, smem, s>>>(a);
-    else k_record_nodes<false><<<a.chunks, kWrThreads, smem, s>>>(a);
-    return cudaGetLastError();
+    const cudaError_t e = launch_early(k_record_count, a.chunks, kRecThreads, 0, 0, s, a);
+    if (e != cudaSuccess) return e;
+    return launch_early(bulk ? k_record_nodes<true> : k_record_nodes<false>, a.chunks, kWrThreads,
+                        smem, 0, s, a);
 }
 
 cudaError_t launch_record_radiance(const RadianceArgs& a, cudaStream_t s) {
     if (a.n == 0) return cudaSuccess;
-    k_record_radiance<<<(a.n + 255) / 256, 256, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_early(k_record_radiance, (a.n + 255) / 256, 256, 0, 0, s, a);
 }
 
 cudaError_t launch_propagate(const NodeView& nb, cudaStream_t s) {
@@ -837,8 +842,7 @@ cudaError_t launch_propagate(const NodeView& nb, cudaStream_t s) {
 }
 
 cudaError_t launch_generate(const GenerateArgs& a, int grid, cudaStream_t s) {
-    k_generate<<<grid, kRecThreads, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_early(k_generate, (unsigned)grid, kRecThreads, 0, 0, s, a);
 }
 
 cudaError_t launch_sample_weights(const WeightArgs& a, cudaStream_t s) {
@@ -848,8 +852,7 @@ cudaError_t launch_sample_weights(const WeightArgs& a, cudaStream_t s) {
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
     const unsigned need = (a.max_n + 255) / 256, cap = (unsigned)sms * 8u;
-    k_sample_weights<<<need < cap ? need : cap, 256, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_early(k_sample_weights, need < cap ? need : cap, 256, 0, 0, s, a);
 }
 
 }  // namespace nrrs

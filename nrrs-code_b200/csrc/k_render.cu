@@ -27,6 +27,7 @@
 #include <vector>
 
 #include "fixed_point.cuh"
+#include "launch_early.cuh"
 #include "nrrs.h"
 
 struct nrrs_scene {
@@ -244,6 +245,7 @@ __device__ __forceinline__ float power_heuristic(float a, float b) {
 // ---- kernels ----
 __global__ void __launch_bounds__(256) k_camera(nrrs_camera c, uint32_t sample, uint32_t seed,
                                                 nrrs_ray_soa r) {
+    wait_for_stream();
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= c.width * c.height) return;
     const V3 fw = normalize(v3(c.forward));
@@ -295,6 +297,7 @@ __device__ __forceinline__ uint32_t ray_key(const nrrs_scene& s, const nrrs_ray_
 __global__ void __launch_bounds__(kSortThreads) k_sort_count(const __grid_constant__ nrrs_scene s,
                                                              nrrs_ray_soa r, const uint32_t* n_dev,
                                                              uint32_t max_n, uint32_t* hist) {
+    wait_for_stream();
     const uint32_t n = min(*n_dev, max_n);
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t warps = gridDim.x * (kSortThreads / 32);
@@ -357,6 +360,7 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_scatter(const __grid_cons
                                                                nrrs_ray_soa r, const uint32_t* n_dev,
                                                                uint32_t max_n, uint32_t* hist,
                                                                uint32_t* order) {
+    wait_for_stream();
     const uint32_t n = min(*n_dev, max_n);
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t warps = gridDim.x * (kSortThreads / 32);
@@ -381,6 +385,7 @@ __global__ void __launch_bounds__(128) k_trace(const __grid_constant__ nrrs_scen
                                                nrrs_ray_soa r, const uint32_t* n_dev,
                                                uint32_t max_n, nrrs_hit_soa h,
                                                const uint32_t* order) {
+    wait_for_stream();
     const uint32_t n = min(*n_dev, max_n);
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const uint32_t i = order ? order[k] : k;
@@ -438,6 +443,7 @@ __global__ void __launch_bounds__(256) k_shade_count(const __grid_constant__ nrr
                                                      const uint32_t* n_dev, uint32_t max_n,
                                                      uint32_t* scratch, uint32_t* n_out,
                                                      uint32_t* n_spec_out) {
+    wait_for_stream();
     __shared__ unsigned s_part[2][8], s_last;
     __shared__ unsigned long long s_w[8];
     const uint32_t n = min(*n_dev, max_n);
@@ -507,6 +513,7 @@ __global__ void __launch_bounds__(256) k_shade(const __grid_constant__ nrrs_scen
                                                uint32_t depth, int64_t* film, float* contrib,
                                                nrrs_path_vertices out, nrrs_path_vertices outs,
                                                int split, const uint32_t* scratch) {
+    wait_for_stream();
     __shared__ unsigned s_warp[2][8];
     const uint32_t n = min(*n_dev, max_n);
     const uint32_t chunks = (max_n + kShadeChunk - 1) / kShadeChunk;
@@ -711,6 +718,7 @@ __global__ void __launch_bounds__(128) k_scatter(const __grid_constant__ nrrs_sc
                                                  const uint32_t* queue, const uint32_t* q_dev,
                                                  uint32_t max_q, uint32_t depth, uint32_t seed,
                                                  nrrs_ray_soa r, nrrs_shadow_soa sh) {
+    wait_for_stream();
     const uint32_t n = min(*q_dev, max_q);
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
         const uint32_t x = queue[j];
@@ -752,6 +760,7 @@ __global__ void __launch_bounds__(128) k_scatter_fixed_rr(const __grid_constant_
 __global__ void __launch_bounds__(128) k_shadow(const __grid_constant__ nrrs_scene s,
                                                 nrrs_shadow_soa sh, const uint32_t* n_dev,
                                                 uint32_t max_n, int64_t* film, float* cout) {
+    wait_for_stream();
     const uint32_t n = min(*n_dev, max_n);
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
         V3 c = v3(sh.contrib + 3 * (size_t)j);
@@ -766,6 +775,7 @@ __global__ void __launch_bounds__(128) k_shadow(const __grid_constant__ nrrs_sce
 
 __global__ void __launch_bounds__(256) k_resolve(const int64_t* film, uint32_t n, float scale,
                                                  float* img) {
+    wait_for_stream();
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
 #pragma unroll
@@ -1040,17 +1050,16 @@ extern "C" int nrrs_camera_rays(const nrrs_camera* c, uint32_t sample, uint32_t 
                                 const nrrs_ray_soa* rays, void* stream) {
     if (!c || !rays || c->width == 0 || c->height == 0) return NRRS_ERR_INVALID_ARG;
     const uint32_t n = c->width * c->height;
-    k_camera<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(*c, sample, seed, *rays);
-    return ok(cudaGetLastError());
+    return ok(launch_early(k_camera, (n + 255) / 256, 256, 0, 0, (cudaStream_t)stream, *c, sample, seed,
+                           *rays));
 }
 
 extern "C" int nrrs_trace(const nrrs_scene* s, const nrrs_ray_soa* rays, const uint32_t* n_dev,
                           uint32_t max_n, const nrrs_hit_soa* hits, void* stream) {
     if (!s || !rays || !n_dev || !hits) return NRRS_ERR_INVALID_ARG;
     if (max_n == 0) return NRRS_OK;
-    k_trace<<<grid_of(max_n, 128, 64), 128, 0, (cudaStream_t)stream>>>(*s, *rays, n_dev, max_n,
-                                                                        *hits, nullptr);
-    return ok(cudaGetLastError());
+    return ok(launch_early(k_trace, grid_of(max_n, 128, 64), 128, 0, 0, (cudaStream_t)stream, *s, *rays,
+                           n_dev, max_n, *hits, nullptr));
 }
 
 extern "C" uint64_t nrrs_trace_scratch_bytes(uint32_t max_n) {
@@ -1072,12 +1081,15 @@ extern "C" int nrrs_trace_sorted(const nrrs_scene* s, const nrrs_ray_soa* rays,
         if (cudaMemsetAsync(hist, 0, 4ull * (kSortBins + 1), st) != cudaSuccess)
             return NRRS_ERR_CUDA;
         const int g = grid_of(max_n, kSortThreads, 8);
-        k_sort_count<<<g, kSortThreads, 0, st>>>(*s, *rays, n_dev, max_n, hist);
-        k_sort_scatter<<<g, kSortThreads, 0, st>>>(*s, *rays, n_dev, max_n, hist, ord);
+        if (launch_early(k_sort_count, g, kSortThreads, 0, 0, st, *s, *rays, n_dev, max_n, hist) !=
+                cudaSuccess ||
+            launch_early(k_sort_scatter, g, kSortThreads, 0, 0, st, *s, *rays, n_dev, max_n, hist,
+                         ord) != cudaSuccess)
+            return NRRS_ERR_CUDA;
         order = ord;
     }
-    k_trace<<<grid_of(max_n, 128, 64), 128, 0, st>>>(*s, *rays, n_dev, max_n, *hits, order);
-    return ok(cudaGetLastError());
+    return ok(launch_early(k_trace, grid_of(max_n, 128, 64), 128, 0, 0, st, *s, *rays, n_dev, max_n,
+                           *hits, order));
 }
 
 extern "C" uint64_t nrrs_shade_scratch_bytes(uint32_t max_n) {
@@ -1104,11 +1116,11 @@ extern "C" int nrrs_shade_split(const nrrs_scene* s, const nrrs_ray_soa* rays,
     uint32_t* sc = static_cast<uint32_t*>(scratch);
     if (cudaMemsetAsync(sc, 0, 4, st) != cudaSuccess) return NRRS_ERR_CUDA;   // the done counter
     const int split = out_specular != nullptr;
-    k_shade_count<<<chunks, 256, 0, st>>>(*s, *rays, *hits, n_dev, max_n, sc, n_out_dev,
-                                          n_specular_dev);
-    k_shade<<<chunks, 256, 0, st>>>(*s, *rays, *hits, n_dev, max_n, depth, film, contrib, *out,
-                                    split ? *out_specular : *out, split, sc);
-    return ok(cudaGetLastError());
+    if (launch_early(k_shade_count, chunks, 256, 0, 0, st, *s, *rays, *hits, n_dev, max_n, sc,
+                     n_out_dev, n_specular_dev) != cudaSuccess)
+        return NRRS_ERR_CUDA;
+    return ok(launch_early(k_shade, chunks, 256, 0, 0, st, *s, *rays, *hits, n_dev, max_n, depth, film,
+                           contrib, *out, split ? *out_specular : *out, split, sc));
 }
 
 extern "C" int nrrs_shade(const nrrs_scene* s, const nrrs_ray_soa* rays, const nrrs_hit_soa* hits,
@@ -1152,9 +1164,8 @@ extern "C" int nrrs_scatter(const nrrs_scene* s, const nrrs_path_vertices* v, co
     if (!s || !v || !rrs_norm || !queue || !queue_size_dev || !rays || !shadow)
         return NRRS_ERR_INVALID_ARG;
     if (max_queue == 0) return NRRS_OK;
-    k_scatter<<<grid_of(max_queue, 128), 128, 0, (cudaStream_t)stream>>>(
-        *s, *v, rrs_norm, queue, queue_size_dev, max_queue, depth, seed, *rays, *shadow);
-    return ok(cudaGetLastError());
+    return ok(launch_early(k_scatter, grid_of(max_queue, 128), 128, 0, 0, (cudaStream_t)stream, *s, *v,
+                           rrs_norm, queue, queue_size_dev, max_queue, depth, seed, *rays, *shadow));
 }
 
 extern "C" int nrrs_scatter_fixed_rr(const nrrs_scene* s, const nrrs_path_vertices* v,
@@ -1174,15 +1185,14 @@ extern "C" int nrrs_trace_shadow(const nrrs_scene* s, const nrrs_shadow_soa* sha
                                  float* contrib_out, void* stream) {
     if (!s || !shadow || !n_dev || !film) return NRRS_ERR_INVALID_ARG;
     if (max_n == 0) return NRRS_OK;
-    k_shadow<<<grid_of(max_n, 128, 64), 128, 0, (cudaStream_t)stream>>>(
-        *s, *shadow, n_dev, max_n, film, contrib_out);
-    return ok(cudaGetLastError());
+    return ok(launch_early(k_shadow, grid_of(max_n, 128, 64), 128, 0, 0, (cudaStream_t)stream, *s,
+                           *shadow, n_dev, max_n, film, contrib_out));
 }
 
 extern "C" int nrrs_film_resolve(const int64_t* film, uint32_t n_pixels, float scale, float* image,
                                  void* stream) {
     if (!film || !image) return NRRS_ERR_INVALID_ARG;
     if (n_pixels == 0) return NRRS_OK;
-    k_resolve<<<(n_pixels + 255) / 256, 256, 0, (cudaStream_t)stream>>>(film, n_pixels, scale, image);
-    return ok(cudaGetLastError());
+    return ok(launch_early(k_resolve, (n_pixels + 255) / 256, 256, 0, 0, (cudaStream_t)stream, film,
+                           n_pixels, scale, image));
 }

@@ -4,6 +4,7 @@
 
 #include <cmath>
 
+#include "launch_early.cuh"
 #include "nrrs_common.cuh"
 
 namespace nrrs {
@@ -167,37 +168,5 @@ struct DeriveArgs {
     uint32_t cell_rows;    // (y, z) rows of the dense levels
 };
 cudaError_t launch_derive(const DeriveArgs& a, int sm_count, cudaStream_t s);
-
-// ---- programmatic stream serialisation: a kernel launched by launch_early is set up while the
-// one before it in the stream finishes; it calls wait_for_stream() before it touches memory
-// (2 to 3 us between the kernels of a step become about 1). `cluster` CTAs per cluster, 0 = none.
-template <class... A>
-cudaError_t launch_early(void (*k)(A...), dim3 grid, unsigned threads, size_t smem, unsigned cluster,
-                         cudaStream_t s, const A&... args) {
-    cudaLaunchConfig_t c{};
-    c.gridDim = grid;
-    c.blockDim = dim3(threads);
-    c.dynamicSmemBytes = smem;
-    c.stream = s;
-    cudaLaunchAttribute at[2]{};
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = cluster;
-    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
-    c.attrs = at;
-    c.numAttrs = cluster ? 2 : 1;
-    const cudaError_t e = cudaLaunchKernelEx(&c, k, args...);
-    if (e != cudaSuccess) cudaGetLastError();   // reported here, not by a later call
-    return e;
-}
-// waits for the kernels before this one in its stream and has their writes visible
-__device__ __forceinline__ void wait_for_stream() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-// lets the next kernel of the stream be set up while this one finishes
-__device__ __forceinline__ void let_next_start() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
 
 }  // namespace nrrs
