@@ -121,14 +121,20 @@ __device__ __forceinline__ bool intersect_v(V3 v0, V3 e1, V3 e2, V3 o, V3 d, flo
     return true;
 }
 
+// 32 aligned bytes in one load
+__device__ __forceinline__ void load8(const float4* p, float4& a, float4& b) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(p));
+}
+
 // a leaf-order triangle of 12 words, read as three 16-byte loads: v0, e1, e2, its input index, and
 // whether it is its leaf's last one
 __device__ __forceinline__ bool intersect_leaf(const float* tri, V3 o, V3 d, float tmax, float bound,
                                                float* t, float* u, float* v, uint32_t* id,
                                                bool* last) {
-    const float4 a = __ldg(reinterpret_cast<const float4*>(tri));
-    const float4 b = __ldg(reinterpret_cast<const float4*>(tri) + 1);
-    const float4 c = __ldg(reinterpret_cast<const float4*>(tri) + 2);
+    const float4* p = reinterpret_cast<const float4*>(tri);
+    const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
     *id = __float_as_uint(c.y);
     *last = __float_as_uint(c.z) != 0;
     return intersect_v({a.x, a.y, a.z}, {a.w, b.x, b.y}, {b.z, b.w, c.x}, o, d, tmax, bound, t, u, v);
@@ -160,7 +166,9 @@ struct Pair {
 };
 __device__ __forceinline__ Pair test_pair(const float4* nodes, int at, V3 o, V3 inv, float tmax) {
     const float4* p = nodes + 2 * (size_t)at;
-    const float4 lo0 = __ldg(p), hi0 = __ldg(p + 1), lo1 = __ldg(p + 2), hi1 = __ldg(p + 3);
+    float4 lo0, hi0, lo1, hi1;
+    load8(p, lo0, hi0);
+    load8(p + 2, lo1, hi1);
     Pair q;
     q.h0 = box_hit(lo0, hi0, o, inv, tmax, &q.t0);
     q.h1 = box_hit(lo1, hi1, o, inv, tmax, &q.t1);
@@ -176,10 +184,11 @@ __device__ __forceinline__ Pair test_pair(const float4* nodes, int at, V3 o, V3 
 // holds a leaf (or the stack is empty), then tests that leaf: lanes of a warp reconverge between
 // the two loops, so the triangle tests run with the warp together.
 // Issue slots (70 %) and L1 (75 %) bound it, with 13 of 32 lanes active. 720p, three depths, the
-// room of 1,000 boxes: 1,240 us with a box per step, 1,137 with a pair. The order by the entered
-// distance takes 1,470 (neighbouring rays go different ways), distances on the stack that drop an
-// entry behind a hit 60 us more, two triangles per leaf 30 more, fused multiply-adds for the slabs
-// 40 more (registers), 12 or 16 CTAs per SM nothing or 110 more.
+// room of 1,000 boxes: 1,240 us with a box per step, 1,137 with a pair in four 16-byte loads, 1,090
+// in two of 32 bytes. The order by the entered distance takes 330 us more (neighbouring rays go
+// different ways), distances on the stack that drop an entry behind a hit 60, the stack in shared
+// memory 15 to 50, two triangles per leaf 30, fused multiply-adds for the slabs 40, 16 CTAs per SM
+// 110; triangles padded to 64 bytes for 32-byte loads take the same.
 __device__ Hit closest_hit(const nrrs_scene& s, V3 o, V3 d, float tmax) {
     Hit h{kMiss, tmax, 0.f, 0.f};   // h.t is the culling bound: tmax until the first hit
     const V3 inv = {1.0f / d.x, 1.0f / d.y, 1.0f / d.z};
@@ -220,8 +229,8 @@ __device__ Hit closest_hit(const nrrs_scene& s, V3 o, V3 d, float tmax) {
 
 // Any hit in (0, tmax), ending at the first triangle hit; pairs as above, the child that is
 // entered first before the other. 720p, three depths: 725 us with a box per step and the far child
-// first (which beat near first there), 510 with pairs in this order, 540 in the order of the axis
-// signs, 660 with the child entered last first.
+// first (which beat near first there), 499 with pairs in this order, 533 in the order of the axis
+// signs, 650 with the child entered last first.
 __device__ bool any_hit(const nrrs_scene& s, V3 o, V3 d, float tmax) {
     const V3 inv = {1.0f / d.x, 1.0f / d.y, 1.0f / d.z};
     const float4* nodes = reinterpret_cast<const float4*>(s.nodes);
