@@ -140,14 +140,29 @@ __device__ __forceinline__ bool intersect_leaf(const float* tri, V3 o, V3 d, flo
     return intersect_v({a.x, a.y, a.z}, {a.w, b.x, b.y}, {b.z, b.w, c.x}, o, d, tmax, bound, t, u, v);
 }
 
-// slab test: the interval of the box along the ray, clipped to [0, tmax]. A 0 x inf product (a
-// ray parallel to a slab, starting on its plane) is NaN, which fminf/fmaxf drop; the box is grown
-// at build time, so such a ray cannot reach a triangle inside it and the miss it gives is right.
-__device__ __forceinline__ bool box_hit(float4 lo, float4 hi, V3 o, V3 inv, float tmax,
+// A ray for slab tests: 1 / d and -o / d, so that a slab's distance is one fused multiply-add,
+// lo / d - o / d. Both are finite for a finite ray: |1 / d| is cut at 2^125 / max(|o|, 1). That
+// ends the interval of an axis with d = 0 at a distance of 2^125 times the box's margin instead of
+// at infinity, and lets no inf - inf through. (A NaN, from an infinite or NaN origin, drops out of
+// fminf and fmaxf: the axis then cuts nothing off.)
+struct SlabRay { V3 inv, off; };
+__device__ __forceinline__ float slab_inv(float d, float o) {
+    const float most = 0x1p125f / fmaxf(fabsf(o), 1.0f);
+    return fminf(fmaxf(1.0f / d, -most), most);
+}
+__device__ __forceinline__ SlabRay slab_ray(V3 o, V3 d) {
+    const V3 inv = {slab_inv(d.x, o.x), slab_inv(d.y, o.y), slab_inv(d.z, o.z)};
+    return {inv, {-o.x * inv.x, -o.y * inv.y, -o.z * inv.z}};
+}
+
+// slab test: the interval of the box along the ray, clipped to [0, tmax]. The roundings of o / d
+// and of the sum are each 6e-8 of |o| and of |lo - o|, which the growth of the boxes covers: it has
+// a part relative to the coordinates and one relative to the scene's extent.
+__device__ __forceinline__ bool box_hit(float4 lo, float4 hi, const SlabRay& r, float tmax,
                                         float* tnear) {
-    const float ax = (lo.x - o.x) * inv.x, bx = (hi.x - o.x) * inv.x;
-    const float ay = (lo.y - o.y) * inv.y, by = (hi.y - o.y) * inv.y;
-    const float az = (lo.z - o.z) * inv.z, bz = (hi.z - o.z) * inv.z;
+    const float ax = __fmaf_rn(lo.x, r.inv.x, r.off.x), bx = __fmaf_rn(hi.x, r.inv.x, r.off.x);
+    const float ay = __fmaf_rn(lo.y, r.inv.y, r.off.y), by = __fmaf_rn(hi.y, r.inv.y, r.off.y);
+    const float az = __fmaf_rn(lo.z, r.inv.z, r.off.z), bz = __fmaf_rn(hi.z, r.inv.z, r.off.z);
     const float t0 = fmaxf(fmaxf(fminf(ax, bx), fminf(ay, by)), fmaxf(fminf(az, bz), 0.f));
     const float t1 = fminf(fminf(fmaxf(ax, bx), fmaxf(ay, by)), fminf(fmaxf(az, bz), tmax));
     *tnear = t0;
@@ -164,34 +179,33 @@ struct Pair {
     int c0, c1, axis;
     bool h0, h1;
 };
-__device__ __forceinline__ Pair test_pair(const float4* nodes, int at, V3 o, V3 inv, float tmax) {
+__device__ __forceinline__ Pair test_pair(const float4* nodes, int at, const SlabRay& r, float tmax) {
     const float4* p = nodes + 2 * (size_t)at;
     float4 lo0, hi0, lo1, hi1;
     load8(p, lo0, hi0);
     load8(p + 2, lo1, hi1);
     Pair q;
-    q.h0 = box_hit(lo0, hi0, o, inv, tmax, &q.t0);
-    q.h1 = box_hit(lo1, hi1, o, inv, tmax, &q.t1);
+    q.h0 = box_hit(lo0, hi0, r, tmax, &q.t0);
+    q.h1 = box_hit(lo1, hi1, r, tmax, &q.t1);
     q.c0 = __float_as_int(lo0.w);
     q.c1 = __float_as_int(lo1.w);
     q.axis = __float_as_int(hi0.w);
     return q;
 }
 
-// Closest hit; ties in t go to the lower input index. A step tests both children of a node (64
-// bytes side by side), goes on with the near one by the sign of the ray on the node's split axis
-// and puts the other on the stack. Each pass of the outer loop first walks down until this lane
-// holds a leaf (or the stack is empty), then tests that leaf: lanes of a warp reconverge between
-// the two loops, so the triangle tests run with the warp together.
-// Issue slots (70 %) and L1 (75 %) bound it, with 13 of 32 lanes active. 720p, three depths, the
+// Closest hit; ties in t go to the lower input index. A lane's step tests both children of a node
+// (64 bytes side by side), goes on with the near one by the sign of the ray on the node's split
+// axis and puts the other on the stack, or it tests a leaf: lanes of a warp do either, and none
+// waits for the others to arrive at leaves.
+// Issue slots and L1 bound it (70 and 75 %), with 13 of 32 lanes active. 720p, three depths, the
 // room of 1,000 boxes: 1,240 us with a box per step, 1,137 with a pair in four 16-byte loads, 1,090
-// in two of 32 bytes. The order by the entered distance takes 330 us more (neighbouring rays go
-// different ways), distances on the stack that drop an entry behind a hit 60, the stack in shared
-// memory 15 to 50, two triangles per leaf 30, fused multiply-adds for the slabs 40, 16 CTAs per SM
-// 110; triangles padded to 64 bytes for 32-byte loads take the same.
+// in two of 32 bytes, 875 without the inner loop that walked every lane to a leaf, 850 with fused
+// multiply-adds for the slabs. The order by the entered distance takes 120 us more (neighbouring
+// rays go different ways), distances on the stack that drop an entry behind a hit 85, the stack in
+// shared memory 35, two triangles per leaf 70, 12 CTAs per SM 17.
 __device__ Hit closest_hit(const nrrs_scene& s, V3 o, V3 d, float tmax) {
     Hit h{kMiss, tmax, 0.f, 0.f};   // h.t is the culling bound: tmax until the first hit
-    const V3 inv = {1.0f / d.x, 1.0f / d.y, 1.0f / d.z};
+    const SlabRay r = slab_ray(o, d);
     const float4* nodes = reinterpret_cast<const float4*>(s.nodes);
     const uint32_t neg = (d.x < 0.f ? 1u : 0u) | (d.y < 0.f ? 2u : 0u) | (d.z < 0.f ? 4u : 0u);
     int stack[kMaxDepth + 1];
@@ -199,11 +213,11 @@ __device__ Hit closest_hit(const nrrs_scene& s, V3 o, V3 d, float tmax) {
     int sp = 1;
     const float4 lo = __ldg(nodes), hi = __ldg(nodes + 1);
     float tn;
-    if (!box_hit(lo, hi, o, inv, h.t, &tn)) return h;
+    if (!box_hit(lo, hi, r, h.t, &tn)) return h;
     int cur = __float_as_int(lo.w);
-    for (;;) {
-        while (cur >= 0) {
-            const Pair q = test_pair(nodes, cur, o, inv, h.t);
+    while (cur != kDone) {
+        if (cur >= 0) {
+            const Pair q = test_pair(nodes, cur, r, h.t);
             if (q.h0 && q.h1) {
                 const bool second = neg >> q.axis & 1u;
                 stack[sp++] = second ? q.c0 : q.c1;
@@ -211,8 +225,8 @@ __device__ Hit closest_hit(const nrrs_scene& s, V3 o, V3 d, float tmax) {
             } else {
                 cur = q.h0 ? q.c0 : q.h1 ? q.c1 : stack[--sp];
             }
+            continue;
         }
-        if (cur == kDone) break;
         bool last;
         for (const float* tri = s.tris + 12 * (size_t)~cur;; tri += 12) {
             float t, u, v;
@@ -229,39 +243,42 @@ __device__ Hit closest_hit(const nrrs_scene& s, V3 o, V3 d, float tmax) {
 
 // Any hit in (0, tmax), ending at the first triangle hit; pairs as above, the child that is
 // entered first before the other. 720p, three depths: 725 us with a box per step and the far child
-// first (which beat near first there), 499 with pairs in this order, 533 in the order of the axis
-// signs, 650 with the child entered last first.
+// first (which beat near first there), 499 with pairs in this order (650 with the child entered last
+// first), 446 without the inner loop (482 in the order of the axis signs), 431 with one pop for
+// both kinds of step (875 -> 884 in the closest hit), 410 with fused multiply-adds.
 __device__ bool any_hit(const nrrs_scene& s, V3 o, V3 d, float tmax) {
-    const V3 inv = {1.0f / d.x, 1.0f / d.y, 1.0f / d.z};
+    const SlabRay r = slab_ray(o, d);
     const float4* nodes = reinterpret_cast<const float4*>(s.nodes);
     int stack[kMaxDepth + 1];
     stack[0] = kDone;
     int sp = 1;
     const float4 lo = __ldg(nodes), hi = __ldg(nodes + 1);
     float tn;
-    if (!box_hit(lo, hi, o, inv, tmax, &tn)) return false;
+    if (!box_hit(lo, hi, r, tmax, &tn)) return false;
     int cur = __float_as_int(lo.w);
-    for (;;) {
-        while (cur >= 0) {
-            const Pair q = test_pair(nodes, cur, o, inv, tmax);
+    while (cur != kDone) {
+        if (cur >= 0) {
+            const Pair q = test_pair(nodes, cur, r, tmax);
             if (q.h0 && q.h1) {
                 const bool second = q.t1 < q.t0;
                 stack[sp++] = second ? q.c0 : q.c1;
                 cur = second ? q.c1 : q.c0;
             } else {
-                cur = q.h0 ? q.c0 : q.h1 ? q.c1 : stack[--sp];
+                cur = q.h0 ? q.c0 : q.c1;
             }
-        }
-        if (cur == kDone) return false;
-        bool last;
-        for (const float* tri = s.tris + 12 * (size_t)~cur;; tri += 12) {
-            float t, u, v;
-            uint32_t id;
-            if (intersect_leaf(tri, o, d, tmax, tmax, &t, &u, &v, &id, &last)) return true;
-            if (last) break;
+            if (q.h0 || q.h1) continue;
+        } else {
+            bool last;
+            for (const float* tri = s.tris + 12 * (size_t)~cur;; tri += 12) {
+                float t, u, v;
+                uint32_t id;
+                if (intersect_leaf(tri, o, d, tmax, tmax, &t, &u, &v, &id, &last)) return true;
+                if (last) break;
+            }
         }
         cur = stack[--sp];
     }
+    return false;
 }
 
 __device__ __forceinline__ void film_add(int64_t* film, uint32_t pixel, V3 c) {
@@ -846,7 +863,7 @@ struct Build {
             }
         }
         // Grow the box so that the slab test never misses a triangle the exact test hits. A slab
-        // distance (lo - o) * inv carries a relative error of about 1.2e-7 of |lo - o|; the margin,
+        // distance lo / d - o / d carries an error of about 1.2e-7 of |lo - o| and 6e-8 of |lo|; the margin,
         // relative to the coordinates and to the scene's extent, stays far above that for ray
         // origins within some 80 scene extents.
         for (int k = 0; k < 3; ++k) {
