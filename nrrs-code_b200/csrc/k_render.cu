@@ -197,8 +197,8 @@ __device__ __forceinline__ Pair test_pair(const float4* nodes, int at, const Sla
 // (64 bytes side by side), goes on with the near one by the sign of the ray on the node's split
 // axis and puts the other on the stack, or it tests a leaf: lanes of a warp do either, and none
 // waits for the others to arrive at leaves.
-// Issue slots and L1 bound it (70 and 75 %), with 13 of 32 lanes active. 720p, three depths, the
-// room of 1,000 boxes: 1,240 us with a box per step, 1,137 with a pair in four 16-byte loads, 1,090
+// L1 (84 %) and issue slots (66 to 72 %) bound it; 28 of 32 lanes are active on camera rays, 15
+// after a bounce. 720p, three depths, the room of 1,000 boxes: 1,240 us with a box per step, 1,137 with a pair in four 16-byte loads, 1,090
 // in two of 32 bytes, 875 without the inner loop that walked every lane to a leaf, 850 with fused
 // multiply-adds for the slabs. The order by the entered distance takes 120 us more (neighbouring
 // rays go different ways), distances on the stack that drop an entry behind a hit 85, the stack in
