@@ -158,14 +158,12 @@ __device__ __forceinline__ SlabRay slab_ray(V3 o, V3 d) {
 // slab test: the interval of the box along the ray, clipped to [0, tmax]. The roundings of o / d
 // and of the sum are each 6e-8 of |o| and of |lo - o|, which the growth of the boxes covers: it has
 // a part relative to the coordinates and one relative to the scene's extent.
-__device__ __forceinline__ bool box_hit(float4 lo, float4 hi, const SlabRay& r, float tmax,
-                                        float* tnear) {
+__device__ __forceinline__ bool box_hit(float4 lo, float4 hi, const SlabRay& r, float tmax) {
     const float ax = __fmaf_rn(lo.x, r.inv.x, r.off.x), bx = __fmaf_rn(hi.x, r.inv.x, r.off.x);
     const float ay = __fmaf_rn(lo.y, r.inv.y, r.off.y), by = __fmaf_rn(hi.y, r.inv.y, r.off.y);
     const float az = __fmaf_rn(lo.z, r.inv.z, r.off.z), bz = __fmaf_rn(hi.z, r.inv.z, r.off.z);
     const float t0 = fmaxf(fmaxf(fminf(ax, bx), fminf(ay, by)), fmaxf(fminf(az, bz), 0.f));
     const float t1 = fminf(fminf(fmaxf(ax, bx), fmaxf(ay, by)), fminf(fmaxf(az, bz), tmax));
-    *tnear = t0;
     return t0 <= t1;
 }
 
@@ -173,9 +171,8 @@ struct Hit { uint32_t prim; float t, u, v; };
 
 constexpr int kDone = INT_MIN;   // below the stack; no leaf's reference
 
-// both children of a node: where the ray enters them and what they are
+// both children of a node: whether the ray enters them and what they are
 struct Pair {
-    float t0, t1;
     int c0, c1, axis;
     bool h0, h1;
 };
@@ -185,8 +182,8 @@ __device__ __forceinline__ Pair test_pair(const float4* nodes, int at, const Sla
     load8(p, lo0, hi0);
     load8(p + 2, lo1, hi1);
     Pair q;
-    q.h0 = box_hit(lo0, hi0, r, tmax, &q.t0);
-    q.h1 = box_hit(lo1, hi1, r, tmax, &q.t1);
+    q.h0 = box_hit(lo0, hi0, r, tmax);
+    q.h1 = box_hit(lo1, hi1, r, tmax);
     q.c0 = __float_as_int(lo0.w);
     q.c1 = __float_as_int(lo1.w);
     q.axis = __float_as_int(hi0.w);
@@ -212,8 +209,7 @@ __device__ Hit closest_hit(const nrrs_scene& s, V3 o, V3 d, float tmax) {
     stack[0] = kDone;
     int sp = 1;
     const float4 lo = __ldg(nodes), hi = __ldg(nodes + 1);
-    float tn;
-    if (!box_hit(lo, hi, r, h.t, &tn)) return h;
+    if (!box_hit(lo, hi, r, h.t)) return h;
     int cur = __float_as_int(lo.w);
     while (cur != kDone) {
         if (cur >= 0) {
@@ -241,26 +237,28 @@ __device__ Hit closest_hit(const nrrs_scene& s, V3 o, V3 d, float tmax) {
     return h;
 }
 
-// Any hit in (0, tmax), ending at the first triangle hit; pairs as above, the child that is
-// entered first before the other. 720p, three depths: 725 us with a box per step and the far child
-// first (which beat near first there), 499 with pairs in this order (650 with the child entered last
-// first), 446 without the inner loop (482 in the order of the axis signs), 431 with one pop for
-// both kinds of step (875 -> 884 in the closest hit), 410 with fused multiply-adds.
+// Any hit in (0, tmax), ending at the first triangle hit; pairs and one loop as above, one pop for
+// both kinds of step (875 -> 884 us in the closest hit, 446 -> 431 here). The far child by the sign
+// on the split axis goes first: a shadow ray starts on a surface, among the boxes it is just
+// leaving, and neighbouring rays share the order. A 720p frame of three depths in a room of 1,000
+// boxes / a 1080p frame of six in a room of 3,000, us: 724 / 2,564 with a box per step in the same
+// order, 510 / 1,893 now; the child that is entered first before the other 408 / 3,178, the one
+// entered last first 487 / 2,925, the longer interval first 459 / 2,531.
 __device__ bool any_hit(const nrrs_scene& s, V3 o, V3 d, float tmax) {
     const SlabRay r = slab_ray(o, d);
+    const uint32_t neg = (d.x < 0.f ? 1u : 0u) | (d.y < 0.f ? 2u : 0u) | (d.z < 0.f ? 4u : 0u);
     const float4* nodes = reinterpret_cast<const float4*>(s.nodes);
     int stack[kMaxDepth + 1];
     stack[0] = kDone;
     int sp = 1;
     const float4 lo = __ldg(nodes), hi = __ldg(nodes + 1);
-    float tn;
-    if (!box_hit(lo, hi, r, tmax, &tn)) return false;
+    if (!box_hit(lo, hi, r, tmax)) return false;
     int cur = __float_as_int(lo.w);
     while (cur != kDone) {
         if (cur >= 0) {
             const Pair q = test_pair(nodes, cur, r, tmax);
             if (q.h0 && q.h1) {
-                const bool second = q.t1 < q.t0;
+                const bool second = !(neg >> q.axis & 1u);
                 stack[sp++] = second ? q.c0 : q.c1;
                 cur = second ? q.c1 : q.c0;
             } else {
