@@ -22,6 +22,8 @@
 //    and reports NRRS_DEV_TIMEOUT. One warp reads 32 predecessor states at a time.
 #include <cooperative_groups.h>
 
+#include <utility>
+
 #include "kernels.hpp"
 
 namespace nrrs {
@@ -568,7 +570,9 @@ __global__ void __launch_bounds__(kDecThreads) k_decide_emit(const __grid_consta
 }
 
 // The whole decision of one segment of up to kSmallSpan x 8 vertices as one cluster of up to 8 CTAs:
-// decide, scan in the CTA, exchange the CTA totals through distributed shared memory, emit. Two
+// decide, scan in the CTA, exchange the CTA totals through distributed shared memory (a CTA stores
+// into another's only after the first cluster barrier, which says that all of them have started; the
+// arrival is at the entry and the wait behind the loads and the scan), emit. Two
 // grids (count, emission) are launch and memory latencies at this size: 3,071 vertices 7.0 us
 // against 7.1 + 3.7 and a gap, 65,536 vertices 7.6 against 7.4 + 3.5. A cluster of 8 is the largest
 // portable one, which sets the bound of 65,536 vertices.
@@ -585,6 +589,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_decide_small(const __grid_con
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const unsigned rank = blockIdx.x;
     unsigned flags = 0;
+    auto started = cluster.barrier_arrive();
     let_next_start();
     wait_for_stream();
     const SegmentTable& S = seg_table(a.segs);
@@ -603,6 +608,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_decide_small(const __grid_con
     }
     if (lane == 31) s_warp[wid] = incl;
     __syncthreads();
+    cluster.barrier_wait(std::move(started));
     if (wid == 0) {
         unsigned w = s_warp[lane];
 #pragma unroll
