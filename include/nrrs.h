@@ -204,7 +204,9 @@ void nrrs_decide_params_default(nrrs_decide_params* p);
 /* ---- inference: replaces prepareInferenceData + inference + "Gen RRS Number"
  *      (network.cpp:297-349, integrator.cpp:1184-1298). Writes the 3 log-statistics
  *      (may be NULL), the clamped factor rrs[n] and, when use_ceil, adds ceil(rrs) to the
- *      context's exact 64-bit normalisation accumulator instead of rrs. ---- */
+ *      context's exact 64-bit normalisation accumulator instead of rrs. On the FP32 path and in
+ *      inference mode 0 of the mixed path, this call and nrrs_infer_accumulate keep nothing in the
+ *      context: they may overlap with each other and with a step on other streams. ---- */
 int nrrs_infer(nrrs_ctx* ctx, const nrrs_vertex_soa* v, uint32_t n,
                const nrrs_decide_params* p, float* stats, float* rrs, void* stream);
 

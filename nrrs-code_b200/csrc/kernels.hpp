@@ -69,7 +69,8 @@ struct InferArgs {
     unsigned long long* ext_acc;  // accumulate into this caller-owned sum instead (sharded)
     const uint8_t* enc_tiles;     // split mode: hash features per tile from k_encode_levels
     uint8_t* x1_tiles;            // split mode 2: RRSNet input per tile ([128 x 16], 4 KB)
-    const float* feat;            // FP32 path: the features of tiles tile_begin .. tile_end - 1
+    // FP32 path: the features of tiles tile_begin .. tile_end - 1 (NULL: the kernel gathers)
+    const float* feat;
     uint32_t tile_begin, tile_end;
 };
 

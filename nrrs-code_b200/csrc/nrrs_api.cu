@@ -222,10 +222,20 @@ int refresh_derived(nrrs_ctx* ctx, cudaStream_t s, bool table = true) {
     return e == cudaSuccess ? NRRS_OK : cuda_fail(ctx, e, "derived images");
 }
 
+// FP32 features of one pass of inference
+struct FeatScratch {
+    float* p = nullptr;
+    uint32_t tiles = 0;
+};
+
+// accumulate: the exact sum goes into the context's scratch, as the steps need it. Only these calls
+// use the context's feature scratch on the FP32 path: they take turns on the context anyway, while
+// the others keep nothing in it and may overlap (the tuner brings a `feat` of its own).
 int run_infer(nrrs_ctx* ctx, const nrrs_vertex_soa* v, const SegmentTable& segs,
               const nrrs_decide_params* p, uint64_t n_total, float* stats, float* rrs,
               bool accumulate, cudaStream_t s, unsigned long long* ext_acc = nullptr,
-              const SegmentTable* resolved = nullptr) {
+              const SegmentTable* resolved = nullptr, FeatScratch feat = {}) {
+    if (accumulate) feat = FeatScratch{ctx->feat, ctx->feat_tiles};
     InferArgs a{};
     a.v = vptrs(v);
     a.enc = ctx->table_h ? half_enc(ctx) : ctx->enc;
@@ -304,25 +314,26 @@ int run_infer(nrrs_ctx* ctx, const nrrs_vertex_soa* v, const SegmentTable& segs,
         return NRRS_OK;
     }
     if (c.precision == NRRS_PREC_FP32) {
-        // encoding and networks in passes that the feature scratch holds
+        // encoding and networks in passes that the feature scratch holds, or one kernel for both
         EncodeF32Args ea{};
         ea.enc = a.enc;
         ea.segs = a.segs;
         ea.pos = a.v.pos;
         ea.table = a.table;
-        ea.out = ctx->feat;
+        ea.out = feat.p;
         ea.tile_stride = kF32TileFloats;
         ea.lane_stride = kTile;
-        a.feat = ctx->feat;
-        for (uint32_t t0 = 0; t0 < segs.total_tiles; t0 += ctx->feat_tiles) {
+        a.feat = feat.p;
+        const uint32_t pass = feat.p ? feat.tiles : segs.total_tiles;
+        for (uint32_t t0 = 0; t0 < segs.total_tiles; t0 += pass) {
             a.tile_begin = ea.tile_begin = t0;
             a.tile_end = ea.tile_end =
-                segs.total_tiles - t0 < ctx->feat_tiles ? segs.total_tiles : t0 + ctx->feat_tiles;
-            {
+                segs.total_tiles - t0 < pass ? segs.total_tiles : t0 + pass;
+            if (feat.p) {
                 ProfScope ps(ctx, NRRS_KERNEL_ENCODE, s);
                 e = launch_encode_f32(ea, ctx->sm_count, s);
+                if (e != cudaSuccess) return cuda_fail(ctx, e, "encoding launch");
             }
-            if (e != cudaSuccess) return cuda_fail(ctx, e, "encoding launch");
             ProfScope ps(ctx, NRRS_KERNEL_INFER_FP32, s);
             e = launch_infer_fp32(a, c.statnet_width, c.statnet_hidden, c.rrsnet_width,
                                   c.rrsnet_hidden, ctx->sm_count, ctx->simt_ctas_per_sm, s);
@@ -1416,6 +1427,12 @@ int nrrs_autotune(nrrs_ctx* ctx, uint32_t n, const char* cache_path, char* repor
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     const bool fp32 = c.precision == NRRS_PREC_FP32;
+    // the FP32 path is timed as the steps run it, with features of the tuner's own
+    FeatScratch feat{nullptr, segs.total_tiles < kF32PassTiles ? segs.total_tiles : kF32PassTiles};
+    if (fp32 && cudaMalloc(&feat.p, sizeof(float) * (size_t)kF32TileFloats * feat.tiles) != cudaSuccess) {
+        feat.p = nullptr;
+        cudaGetLastError();
+    }
     const int saved_ctas = fp32 ? ctx->simt_ctas_per_sm : ctx->tc_ctas_per_sm;
     const int saved_wgs = ctx->tc_wgs, saved_split = ctx->tc_split;
     float best = 1e30f;
@@ -1431,10 +1448,10 @@ int nrrs_autotune(nrrs_ctx* ctx, uint32_t n, const char* cache_path, char* repor
             if (nrrs_set_launch_shape(ctx, k, w) != NRRS_OK) continue;
             int rc = NRRS_OK;
             for (int it = 0; it < 2 && rc == NRRS_OK; ++it)
-                rc = run_infer(ctx, &v, segs, &dp, n, nullptr, rrs, false, 0);
+                rc = run_infer(ctx, &v, segs, &dp, n, nullptr, rrs, false, 0, nullptr, nullptr, feat);
             cudaEventRecord(e0, 0);
             for (int it = 0; it < 5 && rc == NRRS_OK; ++it)
-                rc = run_infer(ctx, &v, segs, &dp, n, nullptr, rrs, false, 0);
+                rc = run_infer(ctx, &v, segs, &dp, n, nullptr, rrs, false, 0, nullptr, nullptr, feat);
             cudaEventRecord(e1, 0);
             if (rc != NRRS_OK || cudaEventSynchronize(e1) != cudaSuccess) continue;
             float ms = 0.f;
@@ -1454,6 +1471,7 @@ int nrrs_autotune(nrrs_ctx* ctx, uint32_t n, const char* cache_path, char* repor
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     cudaFree(d);
+    cudaFree(feat.p);
     nrrs_set_infer_split(ctx, best_split);
     nrrs_set_launch_shape(ctx, best_ctas, best_wgs);
     ctx->tc_pinned = false;   // tuned, not asked for by the caller
