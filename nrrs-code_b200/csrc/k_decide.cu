@@ -424,7 +424,6 @@ __global__ void __launch_bounds__(kDecThreads) k_decide_count(const __grid_const
         __threadfence();
         s_last = atomicAdd(&a.scr->done, 1u) == gridDim.x - 1;
     }
-    let_next_start();
     __syncthreads();
     if (!s_last) return;
     __threadfence();
@@ -735,6 +734,9 @@ cudaError_t launch_decide_context(const DecideArgs& a, cudaStream_t s) {
     const cudaError_t e =
         launch_early(k_decide_count, a.segs.total_tiles, kDecThreads, 0, 0, s, a);
     if (e != cudaSuccess) return e;
+    // The emission is set up as the last CTA of the count leaves. Let in earlier, its CTAs gathered on
+    // the few SMs that were free by then and kept to them: 300,000 vertices scaled up to a budget of
+    // 3 / 12 per vertex took 39 / 92 us with the sum instead of 24 / 33.
     return launch_early(k_decide_emit, a.segs.total_tiles, kDecThreads, 0, 0, s, a);
 }
 
