@@ -629,8 +629,8 @@ __global__ void __launch_bounds__(kSmallThreads) k_decide_small(const __grid_con
 
     uint32_t* q = a.queue + sg.queue_offset + prefix;
     const unsigned room = prefix < sg.queue_capacity ? sg.queue_capacity - prefix : 0u;
-    unsigned pos = thread_excl;
     if (total <= kSmallStage) {
+        unsigned pos = thread_excl;
 #pragma unroll
         for (int j = 0; j < kDecVPT; ++j) {
             if (sv[j] == 0u) continue;  // vertices past the end have no copies
@@ -643,12 +643,49 @@ __global__ void __launch_bounds__(kSmallThreads) k_decide_small(const __grid_con
             else flags |= NRRS_DEV_OVERFLOW;
         }
     } else {
+        // More copies than the stage holds: windows of its size, in which a vertex marks its first
+        // copy's slot with its number in the CTA (they ascend, so a running maximum gives every
+        // slot its vertex). 65,536 vertices scaled up to a budget of 3 / 6 / 12 per vertex:
+        // 14 / 20 / 30 us with the sum, 22 / 35 / 51 with each vertex's thread writing its copies.
+        constexpr unsigned kRows = kSmallStage / kSmallThreads;   // of 32 slots, per warp
+        static_assert(kSmallStage % kSmallThreads == 0, "whole rows");
+        const unsigned first = sg.offset + rank * kSmallSpan;
+        for (unsigned w0 = 0; w0 < total; w0 += kSmallStage) {
+            const unsigned w1 = min(total, w0 + kSmallStage);
+            for (unsigned e = tid; e < kSmallStage; e += kSmallThreads) s_stage[e] = 0u;
+            __syncthreads();
+            unsigned pos = thread_excl;
 #pragma unroll
-        for (int j = 0; j < kDecVPT; ++j)
-            for (unsigned k = 0; k < sv[j]; ++k, ++pos) {
-                if (pos < room) q[pos] = a.sidx ? a.sidx[v0 + j] : v0 + j;
-                else flags |= NRRS_DEV_OVERFLOW;
+            for (int j = 0; j < kDecVPT; ++j) {
+                const unsigned lo = max(pos, w0);
+                pos += sv[j];
+                if (lo < min(pos, w1)) s_stage[lo - w0] = kDecVPT * tid + j + 1;
             }
+            __syncthreads();
+            const unsigned at = wid * kRows * 32 + lane;
+            unsigned row[kRows], most = 0;
+#pragma unroll
+            for (unsigned r = 0; r < kRows; ++r) {
+                row[r] = s_stage[at + r * 32];
+                most = max(most, row[r]);
+            }
+            most = __reduce_max_sync(0xffffffffu, most);
+            if (lane == 0) s_warp[wid] = most;
+            __syncthreads();
+            unsigned last = __reduce_max_sync(0xffffffffu, lane < wid ? s_warp[lane] : 0u);
+#pragma unroll
+            for (unsigned r = 0; r < kRows; ++r) {
+                unsigned x = max(row[r], last);
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1)
+                    x = max(x, __shfl_up_sync(0xffffffffu, x, o));   // lane 0 .. o-1: their own
+                last = __shfl_sync(0xffffffffu, x, 31);
+                const unsigned e = w0 + at + r * 32;
+                if (e < w1 && e < room) q[e] = a.sidx ? a.sidx[first + x - 1] : first + x - 1;
+                else if (e < w1) flags |= NRRS_DEV_OVERFLOW;
+            }
+            __syncthreads();
+        }
     }
     if (flags) atomicOr(&a.scr->status, flags);
 }
@@ -720,8 +757,17 @@ cudaError_t launch_decide(const DecideArgs& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+// The cluster decides a single segment that its 8 CTAs hold, unless many copies are to be expected:
+// the cluster's CTAs emit 8,192 vertices' copies each where the two passes' emit 2,048 vertices'.
+// With the sum, cluster / two passes in us: 65,536 vertices scaled up to a budget of 3 per vertex
+// 14 / 20, 8 25 / 27, 12 30 / 29, 50 84 / 57, 200 224 / 135; up to two chunks of the two passes the
+// cluster is faster however many there are (3,071 vertices, 200 per vertex: 88 / 121).
 int decide_launches(const DecideArgs& a) {
-    return a.segs.n == 1 && a.segs.s[0].count <= 8 * kSmallSpan ? 1 : 2;
+    const Segment& sg = a.segs.s[0];
+    if (a.segs.n != 1 || sg.count > 8 * kSmallSpan) return 2;
+    if (sg.count <= 2 * kDecChunk) return 1;
+    const double kept = (double)a.clamp_max * sg.count;
+    return (a.scale_up ? sg.budget : fmin(kept, sg.budget)) <= 8.0 * sg.count ? 1 : 2;
 }
 
 cudaError_t launch_decide_context(const DecideArgs& a, cudaStream_t s) {

@@ -41,6 +41,7 @@ struct DecideArgs {
     float normalize_rate;
     int32_t use_ceil;
     int32_t scale_up;
+    float clamp_max;              // of the factors (the host's estimate of the copies)
     double inv_fixed_scale;
     uint32_t spin_limit;
     int32_t split_chunked;        // two-pass decision: split is scratch with one block per chunk

@@ -390,6 +390,7 @@ int run_decide(nrrs_ctx* ctx, const float* rrs, const float* rnd, const uint32_t
     d.normalize_rate = p->normalize_rate;
     d.use_ceil = p->use_ceil;
     d.scale_up = p->scale_up;
+    d.clamp_max = p->clamp_max;
     d.inv_fixed_scale = 1.0 / fp.fixed_scale;
     d.spin_limit = 1u << 22;
     if (d.segs.total_tiles > ctx->max_chunks)
