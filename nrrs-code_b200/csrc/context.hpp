@@ -77,6 +77,7 @@ struct nrrs_ctx {
     // training scratch
     void* train_scratch = nullptr;
     size_t train_scratch_bytes = 0;
+    bool train_compact = false;  // FP32 training in the smaller scratch (train_scratch_bytes)
     double* loss_dev = nullptr;  // [2] last losses
     double* loss_sums = nullptr; // batch sums of the loss weights (launch_loss_sums' block)
 
@@ -89,7 +90,7 @@ struct nrrs_ctx {
     int train_split = 1;         // training mode of the tcgen05 path: 0 fused, 1 split
     uint8_t* enc_tiles = nullptr;  // split mode: hash-feature tiles (kEncTileBytes each)
     uint32_t enc_tiles_cap = 0;
-    float* feat = nullptr;         // FP32 path: hash features of one inference pass
+    float* feat = nullptr;         // FP32 path: hash features of one pass of a step (may be null)
     uint32_t feat_tiles = 0;       // its tiles
     uint8_t* x1_tiles = nullptr;   // split mode 2: RRSNet input tiles (kX1TileBytes each)
     nrrs::Profiler prof;
@@ -153,7 +154,10 @@ cudaError_t launch_scatter_table(nrrs_ctx* ctx, const float* pos, uint32_t n, co
                                  cudaStream_t s);
 // Adam on ctx->grads scaled by `scale` (copied in from grads_dev first when it is not ctx->grads)
 cudaError_t launch_adam_step(nrrs_ctx* ctx, bool train_rrs, cudaStream_t s, float scale = 1.0f);
-size_t train_scratch_bytes(const nrrs_config& cfg, uint32_t n, int sm_count);
+// compact: the FP32 step's smaller layout, in which the lane gradients lie in rows of the RRSNet
+// deltas (so the scatter is over before the RRSNet kernel) and a weight-gradient chunk has at least
+// 2,048 samples
+size_t train_scratch_bytes(const nrrs_config& cfg, uint32_t n, int sm_count, bool compact);
 // the tensor-core training step covers 64-wide networks in mixed precision
 bool train_tc_supported(const nrrs_config& cfg);
 }  // namespace nrrs

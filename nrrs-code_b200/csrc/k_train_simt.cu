@@ -687,15 +687,17 @@ __global__ void __launch_bounds__(kWThr, 2) k_wgrad(const __grid_constant__ WGra
 
 // samples per weight-gradient chunk of an n-sample step: 256 chunks (times the layers: several
 // waves of the grid, so that the last one costs little), and at least 256 samples to each, four
-// stages, so that a chunk's start-up and its partial stay small beside it
-uint32_t wgrad_chunk(uint64_t n) {
+// stages, so that a chunk's start-up and its partial stay small beside it (2,048 in the compact
+// layout, for fewer partials)
+uint32_t wgrad_chunk(uint64_t n, bool compact) {
+    const uint64_t least = compact ? 2048 : 256;
     uint64_t c = (n + 255) / 256;
     c = (c + kWS - 1) / kWS * kWS;
-    return (uint32_t)(c < 256 ? 256 : c);
+    return (uint32_t)(c < least ? least : c);
 }
 // chunk partials that steps of up to n samples need
-uint64_t wgrad_chunks_max(uint64_t n) {
-    const uint64_t c = (n + 255) / 256;
+uint64_t wgrad_chunks_max(uint64_t n, bool compact) {
+    const uint64_t least = compact ? 2048 : 256, c = (n + least - 1) / least;
     return c < 256 ? c : 256;
 }
 
@@ -895,18 +897,19 @@ struct Layout {
     uint32_t r_x0, r_hs, r_dhs, r_dx, r_dy, r_x1, r_hr, r_dhr, r_draw, rows;
 };
 
-Layout layout_of(const nrrs_config& c) {
+Layout layout_of(const nrrs_config& c, bool compact) {
     Layout L{};
     uint32_t r = 0;
     const bool ref = c.network == NRRS_NET_REFERENCE;
     L.r_x0 = r; r += ref ? kRefStatIn : 56;
     L.r_hs = r; r += c.statnet_hidden * c.statnet_width;
     L.r_dhs = r; r += c.statnet_hidden * c.statnet_width;
-    L.r_dx = r; r += 2 * c.n_levels;
+    L.r_dx = r; r += compact ? 0 : 2 * c.n_levels;
     L.r_dy = r; r += ref ? 8 : 4;
     L.r_x1 = r; r += 16;
     L.r_hr = r; r += c.rrsnet_hidden * c.rrsnet_width;
-    L.r_dhr = r; r += c.rrsnet_hidden * c.rrsnet_width;
+    L.r_dhr = r; r += c.rrsnet_hidden * c.rrsnet_width;   // at least 2 * n_levels rows
+    if (compact) L.r_dx = L.r_dhr;
     L.r_draw = r; r += 4;
     L.rows = r;
     return L;
@@ -969,14 +972,14 @@ size_t train_tc_scratch_bytes(const nrrs_config& c, uint32_t n, int sm_count);
 int train_step_tc(nrrs_ctx* ctx, const VertexPtrs& v, const float* target, uint32_t n,
                   double* loss_dev, cudaStream_t s, bool apply, const LossWeights* lw);
 
-size_t train_scratch_bytes(const nrrs_config& c, uint32_t n, int sm_count) {
+size_t train_scratch_bytes(const nrrs_config& c, uint32_t n, int sm_count, bool compact) {
     if (train_tc_supported(c)) return train_tc_scratch_bytes(c, n, sm_count);
-    const Layout L = layout_of(c);
+    const Layout L = layout_of(c, compact);
     const uint64_t mlp = (uint64_t)64 * c.statnet_width + (uint64_t)(c.statnet_hidden - 1) *
                          c.statnet_width * c.statnet_width + 3ull * c.statnet_width +
                          16ull * c.rrsnet_width + (uint64_t)(c.rrsnet_hidden - 1) * c.rrsnet_width *
                          c.rrsnet_width + (uint64_t)c.rrsnet_width;
-    const uint64_t chunks = wgrad_chunks_max(n);
+    const uint64_t chunks = wgrad_chunks_max(n, compact);
     return sizeof(float) * (uint64_t)L.rows * ld_of(n) + sizeof(double) * 4 * (uint64_t)sm_count * 16 +
            sizeof(float) * chunks * mlp + 1024;
 }
@@ -986,9 +989,9 @@ int train_step_impl(nrrs_ctx* ctx, const VertexPtrs& v, const float* target, uin
     if (train_tc_supported(ctx->cfg))
         return train_step_tc(ctx, v, target, n, loss_dev, s, apply, lw);
     const nrrs_config& c = ctx->cfg;
-    const Layout L = layout_of(c);
+    const Layout L = layout_of(c, ctx->train_compact);
     const uint32_t ld = ld_of(c.max_train);
-    const uint32_t chunk = wgrad_chunk(n);
+    const uint32_t chunk = wgrad_chunk(n, ctx->train_compact);
     const uint64_t chunks = (n + chunk - 1) / chunk;
     const uint64_t mlp = ctx->n_stat + ctx->n_rrs;
     uint8_t* base = reinterpret_cast<uint8_t*>(ctx->train_scratch);
@@ -1053,15 +1056,17 @@ int train_step_impl(nrrs_ctx* ctx, const VertexPtrs& v, const float* target, uin
     // The scatter is bound by L2 reductions, the RRSNet kernel and the weight gradients by the
     // FP32 pipe: it runs beside them on the context's side stream, forked after the StatNet
     // kernel and joined before Adam (nothing in between reads the table gradient).
+    // (In the compact layout the RRSNet kernel overwrites the lane gradients: the scatter stays on
+    // the caller's stream.)
     bool forked = false;
     auto after_stat = [&]() -> cudaError_t {
+        const LaneGrads g{act + (size_t)L.r_dx * ld, 2 * (size_t)ld, 1, ld, 1.0f};
+        if (ctx->train_compact) return launch_scatter_table(ctx, v.pos, n, g, s);
         cudaError_t ef = cudaEventRecord(ctx->ev_fork, s);
         if (ef == cudaSuccess) ef = cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0);
         if (ef != cudaSuccess) return ef;
         forked = true;
-        ef = launch_scatter_table(ctx, v.pos, n,
-                                  LaneGrads{act + (size_t)L.r_dx * ld, 2 * (size_t)ld, 1, ld, 1.0f},
-                                  ctx->side);
+        ef = launch_scatter_table(ctx, v.pos, n, g, ctx->side);
         const cudaError_t ej = cudaEventRecord(ctx->ev_join, ctx->side);
         return ef != cudaSuccess ? ef : ej;
     };

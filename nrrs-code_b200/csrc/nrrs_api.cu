@@ -645,12 +645,6 @@ int nrrs_create(const nrrs_config* cfg, nrrs_ctx** out) {
         if (ctx->table_h) NRRS_ALLOC(ctx->table_h_inf, half_table_bytes(ctx));
         if (ctx->cells) NRRS_ALLOC(ctx->cells_inf, 32 * (size_t)ctx->n_cells);
     }
-    if (c.precision == NRRS_PREC_FP32) {
-        // a batched call's segments are padded to whole tiles
-        const uint32_t tiles = (c.max_queue + kTile - 1) / kTile + kMaxSegments;
-        ctx->feat_tiles = tiles < kF32PassTiles ? tiles : kF32PassTiles;
-        NRRS_ALLOC(ctx->feat, sizeof(float) * (size_t)kF32TileFloats * ctx->feat_tiles);
-    }
     if (train_tc_supported(c))
         NRRS_ALLOC(ctx->tpack, train_pack_bytes(c.statnet_width, c.statnet_hidden,
                                                 c.rrsnet_width, c.rrsnet_hidden));
@@ -661,9 +655,27 @@ int nrrs_create(const nrrs_config* cfg, nrrs_ctx** out) {
     NRRS_ALLOC(ctx->loss_dev, sizeof(double) * 2);
     NRRS_ALLOC(ctx->segs_dev, sizeof(SegmentTable) * 2);
     NRRS_ALLOC(ctx->loss_sums, sizeof(double) * kLossSumDoubles);
-    ctx->train_scratch_bytes = train_scratch_bytes(c, c.max_train, ctx->sm_count);
-    NRRS_ALLOC(ctx->train_scratch, ctx->train_scratch_bytes);
+    // The FP32 path's scratch for speed alone is taken where the device has room: the training step's
+    // own rows for the lane gradients and its finer weight-gradient chunks, then the features of a
+    // step. A smaller device, or a full one, holds a context without them.
+    ctx->train_scratch_bytes = train_scratch_bytes(c, c.max_train, ctx->sm_count, false);
+    if (cudaMalloc(&ctx->train_scratch, ctx->train_scratch_bytes) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->train_compact = true;
+        ctx->train_scratch_bytes = train_scratch_bytes(c, c.max_train, ctx->sm_count, true);
+        NRRS_ALLOC(ctx->train_scratch, ctx->train_scratch_bytes);
+    }
 #undef NRRS_ALLOC
+    if (c.precision == NRRS_PREC_FP32) {
+        // a batched call's segments are padded to whole tiles
+        const uint32_t tiles = (c.max_queue + kTile - 1) / kTile + kMaxSegments;
+        ctx->feat_tiles = tiles < kF32PassTiles ? tiles : kF32PassTiles;
+        if (cudaMalloc(&ctx->feat, sizeof(float) * (size_t)kF32TileFloats * ctx->feat_tiles) !=
+            cudaSuccess) {
+            cudaGetLastError();
+            ctx->feat = nullptr;   // the steps' inference kernel gathers for itself
+        }
+    }
 
     // parameters: table ~ U(-s, s), MLPs Xavier-uniform (seeded, host side)
     std::vector<float> h(ctx->n_params);
