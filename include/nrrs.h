@@ -365,8 +365,9 @@ int nrrs_get_device_status(nrrs_ctx* ctx, uint32_t* flags, void* stream);
  *      the context and, with a cache path, reuses or records the choice in a JSON file keyed by
  *      device name, network shape and precision. report (may be NULL) receives a JSON summary.
  *      Synchronous. Short queues of the tcgen05 path (one wave of 32 vertices per CTA) run a kernel
- *      of their own, with the same bits, unless the caller chose a shape or mode with the setters
- *      below. ---- */
+ *      of their own, with the same bits, unless the caller chose a shape or a mode other than 0
+ *      with the setters below; nrrs_set_infer_split(ctx, 0) takes the mode back, nrrs_autotune
+ *      both. ---- */
 int nrrs_autotune(nrrs_ctx* ctx, uint32_t n, const char* cache_path, char* report,
                   size_t report_len);
 int nrrs_set_launch_shape(nrrs_ctx* ctx, int32_t ctas_per_sm, int32_t warpgroups);

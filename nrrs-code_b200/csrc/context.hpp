@@ -85,7 +85,8 @@ struct nrrs_ctx {
     int tc_ctas_per_sm = 0;      // autotuned occupancy of the tcgen05 kernel (0 = default)
     int tc_wgs = 1;              // autotuned warpgroups per CTA of the tcgen05 kernel (1 or 2)
     int simt_ctas_per_sm = 0;    // autotuned occupancy of the FP32 kernel (0 = default)
-    bool tc_pinned = false;      // the caller chose shape or mode: short queues keep to them too
+    // the caller chose a shape, or a mode other than the default: short queues keep to it too
+    bool shape_pinned = false, mode_pinned = false;
     int tc_split = 0;            // inference mode of the tcgen05 path: 0 fused, 1 split
     int train_split = 1;         // training mode of the tcgen05 path: 0 fused, 1 split
     uint8_t* enc_tiles = nullptr;  // split mode: hash-feature tiles (kEncTileBytes each)

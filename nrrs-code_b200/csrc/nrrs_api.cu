@@ -258,7 +258,7 @@ int run_infer(nrrs_ctx* ctx, const nrrs_vertex_soa* v, const SegmentTable& segs,
     cudaError_t e;
     if (segs.total_tiles == 0) return NRRS_OK;
     const int split = c.precision != NRRS_PREC_FP32 ? ctx->tc_split : 0;
-    if (c.precision != NRRS_PREC_FP32 && !ctx->tc_pinned &&
+    if (c.precision != NRRS_PREC_FP32 && !ctx->shape_pinned && !ctx->mode_pinned &&
         infer_small_fits(segs, c.statnet_width, c.statnet_hidden, ctx->sm_count)) {
         {
             ProfScope ps(ctx, NRRS_KERNEL_INFER_TC, s);
@@ -1254,7 +1254,7 @@ int nrrs_set_launch_shape(nrrs_ctx* ctx, int32_t ctas_per_sm, int32_t warpgroups
         return fail(ctx, NRRS_ERR_UNSUPPORTED, "launch shape not available for this network");
     ctx->tc_ctas_per_sm = ctas_per_sm;
     ctx->tc_wgs = warpgroups;
-    ctx->tc_pinned = true;
+    ctx->shape_pinned = true;
     return NRRS_OK;
 }
 
@@ -1284,7 +1284,7 @@ int nrrs_set_infer_split(nrrs_ctx* ctx, int32_t split) {
         ctx->enc_tiles_cap = cap;
     }
     ctx->tc_split = split;
-    ctx->tc_pinned = true;
+    ctx->mode_pinned = split != 0;
     // the warpgroup count must exist in the new mode
     if (infer_max_ctas(c.statnet_width, c.statnet_hidden, c.rrsnet_width, c.rrsnet_hidden,
                        c.precision, ctx->tc_wgs, split) <= 0)
@@ -1395,7 +1395,7 @@ int nrrs_autotune(nrrs_ctx* ctx, uint32_t n, const char* cache_path, char* repor
     int ctas = 0, wgs = 1, split = 0;
     if (cache_path && cache_lookup(cache_path, key, &ctas, &wgs, &split) &&
         nrrs_set_infer_split(ctx, split) == NRRS_OK && nrrs_set_launch_shape(ctx, ctas, wgs) == NRRS_OK) {
-        ctx->tc_pinned = false;
+        ctx->shape_pinned = ctx->mode_pinned = false;
         rep << "{\"key\": \"" << key << "\", \"cached\": [" << ctas << ", " << wgs << ", " << split
             << "]}";
         if (report && report_len) std::snprintf(report, report_len, "%s", rep.str().c_str());
@@ -1487,7 +1487,7 @@ int nrrs_autotune(nrrs_ctx* ctx, uint32_t n, const char* cache_path, char* repor
     cudaFree(feat.p);
     nrrs_set_infer_split(ctx, best_split);
     nrrs_set_launch_shape(ctx, best_ctas, best_wgs);
-    ctx->tc_pinned = false;   // tuned, not asked for by the caller
+    ctx->shape_pinned = ctx->mode_pinned = false;   // tuned, not asked for by the caller
     rep << "], \"best\": [" << best_ctas << ", " << best_wgs << ", " << best_split
         << "], \"best_ms\": " << best << "}";
     if (cache_path) cache_store(cache_path, key, best_ctas, best_wgs, best_split);
