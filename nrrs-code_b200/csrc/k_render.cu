@@ -20,6 +20,7 @@
 // A C restatement of the same steps (brute-force intersection instead of the BVH) checks the
 // kernels bit for bit.
 #include <algorithm>
+#include <cfloat>
 #include <climits>
 #include <cmath>
 #include <cstring>
@@ -143,11 +144,12 @@ __device__ __forceinline__ bool intersect_leaf(const float* tri, V3 o, V3 d, flo
 // A ray for slab tests: 1 / d and -o / d, so that a slab's distance is one fused multiply-add,
 // lo / d - o / d. Both are finite for a finite ray: |1 / d| is cut at 2^125 / max(|o|, 1). That
 // ends the interval of an axis with d = 0 at a distance of 2^125 times the box's margin instead of
-// at infinity, and lets no inf - inf through. (A NaN, from an infinite or NaN origin, drops out of
-// fminf and fmaxf: the axis then cuts nothing off.)
+// at infinity, and lets no inf - inf through. An infinite origin keeps 1 / d above zero, so that
+// -o / d is infinite and the ray ends at the root (as a NaN, which drops out of fminf and fmaxf, the
+// axis cut nothing off, and the ray visited every leaf). A NaN origin cuts nothing off.
 struct SlabRay { V3 inv, off; };
 __device__ __forceinline__ float slab_inv(float d, float o) {
-    const float most = 0x1p125f / fmaxf(fabsf(o), 1.0f);
+    const float most = 0x1p125f / fminf(fmaxf(fabsf(o), 1.0f), FLT_MAX);
     return fminf(fmaxf(1.0f / d, -most), most);
 }
 __device__ __forceinline__ SlabRay slab_ray(V3 o, V3 d) {
