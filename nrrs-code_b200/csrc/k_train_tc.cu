@@ -390,8 +390,12 @@ __global__ void __launch_bounds__(128 * WGS, 1) k_ttc_stat(const __grid_constant
 // FP32 table-gradient bytes per scatter launch (a fraction of L2): 20 MB beside the mixed step's
 // kernels (64 x 2, 2^19 entries, 262,144 samples: 472 us a step, 477 with 40 MB, 493 with 72, 468
 // with 10; at 2^22 entries a level is 34 MB anyway), 40 MB beside the FP32 step's, which leave few
-// SM slots to start launches in (1,017 us; 1,030 with 20 MB, 1,055 with 10, 1,022 with 72)
+// SM slots to start launches in (1,017 us; 1,030 with 20 MB, 1,055 with 10, 1,022 with 72). An FP32
+// step of few samples reads few zeros back, and its launches are what it waits for: one group (64 x 2,
+// 2^22 entries, 1 / 4,096 / 16,384 samples: 524 / 546 / 592 us a step, 596 / 603 / 639 in 16 groups;
+// 65,536 842 / 828).
 constexpr uint64_t kScatterGroupTc = 20ull << 20, kScatterGroupFp32 = 40ull << 20;
+constexpr uint32_t kScatterFewFp32 = 16384;
 
 struct ScatterLvArgs {
     EncodeParams enc;
@@ -885,7 +889,9 @@ cudaError_t launch_scatter_table(nrrs_ctx* ctx, const float* pos, uint32_t n, co
     const uint32_t g_max =
         (uint32_t)(ctx->sm_count * resident_ctas((const void*)k_scatter_levels, 128, 0, 16));
     const int nl = ctx->cfg.n_levels;
-    const uint64_t group_bytes = train_tc_supported(ctx->cfg) ? kScatterGroupTc : kScatterGroupFp32;
+    const uint64_t group_bytes = train_tc_supported(ctx->cfg) ? kScatterGroupTc
+                                 : n <= kScatterFewFp32      ? ~0ull
+                                                             : kScatterGroupFp32;
     auto level_rows = [&](int l) -> uint64_t {
         const LevelDev& lv = ctx->enc.lv[l];
         const uint64_t r = (uint64_t)lv.res + 1;
