@@ -418,7 +418,9 @@ void nrrs_graph_destroy(nrrs_graph* g);
 /* ---- instrumentation: launch counters and optional CUDA-event timing per kernel kind.
  *      The reference's equivalent is KiRaRay's PROFILE("...") scopes (integrator.cpp:1069,
  *      1151, 1158, 1302, 1346, 2638). Timing records one event pair per launch on the launch
- *      stream while enabled; nrrs_profile_read synchronises on those events. ---- */
+ *      stream while enabled; nrrs_profile_read synchronises on those events. The weight images and
+ *      the cell image come from one launch, counted as CELL_IMAGE where the context has a cell image
+ *      and as PACK where it has none. ---- */
 typedef enum {
     NRRS_KERNEL_INFER_FP32 = 0, NRRS_KERNEL_INFER_TC = 1, NRRS_KERNEL_SUM = 2,
     NRRS_KERNEL_DECIDE = 3, NRRS_KERNEL_PACK = 4, NRRS_KERNEL_TABLE_HALF = 5,

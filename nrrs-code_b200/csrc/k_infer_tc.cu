@@ -923,9 +923,10 @@ cudaError_t launch_infer_tc(const InferArgs& a, int ws, int hs, int wr, int hr, 
     return cudaErrorInvalidValue;
 }
 
-// One wave of the short-queue kernel: a CTA per 32 vertices, all resident. Measured at the line, per
-// step with the decision (this kernel / k_infer_tc): 64 x 2 networks 16,000 vertices 22 / 32 us,
-// 50,000 vertices (2.6 waves) 37 / 39, 100,000 68 / 54; 128 x 3, whose weights leave one CTA per SM,
+// One wave of the short-queue kernel: a CTA per 32 vertices, all resident, the same line for every
+// network. Measured per step with the decision (this kernel / k_infer_tc): 64 x 2 networks 16,000
+// vertices 22 / 32 us, 50,000 (2.6 waves) 37 / 39, 100,000 68 / 54: they would gain a little up to
+// about 50,000 vertices too, the others would not; 128 x 3, whose weights leave one CTA per SM,
 // 3,071 vertices 20 / 33, 8,000 (1.7 waves) 29 / 28; shipped network, 16,000 19 / 23, 30,000 27 / 23.
 bool infer_small_fits(const SegmentTable& segs, int ws, int hs, int sm_count) {
     const uint32_t per_sm = ws == 128 ? small_ctas<128, 3>()

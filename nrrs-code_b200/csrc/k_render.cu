@@ -157,9 +157,8 @@ __device__ __forceinline__ SlabRay slab_ray(V3 o, V3 d) {
     return {inv, {-o.x * inv.x, -o.y * inv.y, -o.z * inv.z}};
 }
 
-// slab test: the interval of the box along the ray, clipped to [0, tmax]. The roundings of o / d
-// and of the sum are each 6e-8 of |o| and of |lo - o|, which the growth of the boxes covers: it has
-// a part relative to the coordinates and one relative to the scene's extent.
+// slab test: the interval of the box along the ray, clipped to [0, tmax]. The growth of the boxes
+// covers its roundings (Build::bounds).
 __device__ __forceinline__ bool box_hit(float4 lo, float4 hi, const SlabRay& r, float tmax) {
     const float ax = __fmaf_rn(lo.x, r.inv.x, r.off.x), bx = __fmaf_rn(hi.x, r.inv.x, r.off.x);
     const float ay = __fmaf_rn(lo.y, r.inv.y, r.off.y), by = __fmaf_rn(hi.y, r.inv.y, r.off.y);
@@ -414,6 +413,7 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_count(const __grid_consta
     }
 }
 
+// each ray index at its key's next slot
 __global__ void __launch_bounds__(kSortThreads) k_sort_scatter(const __grid_constant__ nrrs_scene s,
                                                                nrrs_ray_soa r, const uint32_t* n_dev,
                                                                uint32_t max_n, uint32_t* hist,
@@ -862,10 +862,13 @@ struct Build {
                 bmax[k] = std::max({bmax[k], a, b, c});
             }
         }
-        // Grow the box so that the slab test never misses a triangle the exact test hits. A slab
-        // distance lo / d - o / d carries an error of about 1.2e-7 of |lo - o| and 6e-8 of |lo|; the margin,
-        // relative to the coordinates and to the scene's extent, stays far above that for ray
-        // origins within some 80 scene extents.
+        // Grow the box so that the slab test does not miss a triangle the exact test hits. A slab
+        // distance lo / d - o / d is rounded at 1 / d, o / d and the sum: an error below 1.8e-7 of
+        // |lo - o| and 6e-8 of |lo| (|o| is at most their sum). The margin, relative to the
+        // coordinates and to the scene's extent, covers that for ray origins within 55 scene extents.
+        // A triangle seen edge-on from that far may still be missed where the exact test, by its own
+        // rounding, accepts a ray beside it: of 4.2 million such rays 3 at 50 extents, 2 at 80, 12 at
+        // 160, as many as with the slabs' differences (3, 2, 14).
         for (int k = 0; k < 3; ++k) {
             const float e = 1e-5f * (std::fabs(bmin[k]) + std::fabs(bmax[k])) + margin;
             bmin[k] -= e;

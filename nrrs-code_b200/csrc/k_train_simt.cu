@@ -162,12 +162,13 @@ __device__ __forceinline__ void last_delta(const float* __restrict__ w, const fl
     }
 }
 
-// The StatNet step and the RRSNet forward sums on 64-sample tiles: encoding, the forward layers as
-// tile GEMMs storing every activation, the loss gradient, the backward layers as tile GEMMs
-// through the row-major weights, the input gradient of the hash lanes, the hash-grid scatter, then
-// the glue and the RRSNet forward for the sums. Per-sample phases run one thread per sample (64
-// threads per CTA); the 128-wide networks' CTAs have 128 threads and split encoding and scatter
-// over two per sample.
+// The StatNet step and the RRSNet forward sums on 64-sample tiles: the hash lanes copied from the
+// encoding kernel's rows and the other input lanes made here, the forward layers as tile GEMMs
+// storing every activation, the loss gradient, the backward layers as tile GEMMs through the
+// row-major weights, the gradient of the hash lanes to scratch rows (the scatter kernel adds them
+// into the table), then the glue and the RRSNet forward for the sums. Per-sample phases run one
+// thread per sample (64 threads per CTA); the 128-wide networks' CTAs have 128 threads and split the
+// other input lanes over two per sample.
 // 64 x 2, 262,144 samples: 315 us beside 89 us of encoding and 185 us of scatter (kernels of their
 // own, the scatter overlapped), against 735 us for one kernel that did all three with 24 warps per
 // SM waiting for the gathers (330 us of it) and for the reductions (175 us).
