@@ -331,14 +331,25 @@ __device__ __forceinline__ uint8_t* split_of_chunk(const DecideArgs& a, unsigned
     return a.split_chunked ? a.split + (size_t)c * kDecChunk : a.split + first;
 }
 
+// whether the kDecVPT vertices from v0 on are read and stored in whole words
+__device__ __forceinline__ bool whole_run(const DecideArgs& a, unsigned v0, unsigned end) {
+    return v0 + kDecVPT <= end && ((reinterpret_cast<uintptr_t>(a.rrs + v0) |
+                                    reinterpret_cast<uintptr_t>(a.rnd + v0)) & 15u) == 0;
+}
+// the split bytes of vertices 4 g .. 4 g + 3 of a run, as they are stored: a factor of -1 or less has a
+// count above 255, whose upper bytes fall on its neighbours where whole words are stored
+__device__ __forceinline__ uint32_t split_word(const unsigned (&sv)[kDecVPT], int g, bool whole) {
+    const unsigned m = whole ? ~0u : 255u;
+    return (sv[4 * g] & m) | (sv[4 * g + 1] & m) << 8 | (sv[4 * g + 2] & m) << 16 |
+           sv[4 * g + 3] << 24;
+}
+
 // Decision of the kDecVPT consecutive vertices v0 .. (those below `end`) of segment sg: rrs_norm,
 // and the split counts into sv and, where cs is not null, to cs[0 ..]. Returns their sum.
 __device__ __forceinline__ unsigned decide_run(const DecideArgs& a, float scale, unsigned v0,
                                                unsigned end, uint8_t* cs, unsigned (&sv)[kDecVPT],
                                                unsigned* flags) {
-    const bool vec = v0 + kDecVPT <= end &&
-                     ((reinterpret_cast<uintptr_t>(a.rrs + v0) |
-                       reinterpret_cast<uintptr_t>(a.rnd + v0)) & 15u) == 0;
+    const bool vec = whole_run(a, v0, end);
     constexpr int kQ = kDecVPT / 4;
     float rv[kDecVPT], nv[kDecVPT];
     if (vec) {
@@ -384,12 +395,11 @@ __device__ __forceinline__ unsigned decide_run(const DecideArgs& a, float scale,
         }
         if (cs && (reinterpret_cast<uintptr_t>(cs) & 3u) == 0) {
 #pragma unroll
-            for (int g = 0; g < kQ; ++g)
-                reinterpret_cast<uint32_t*>(cs)[g] = sv[4 * g] | sv[4 * g + 1] << 8 |
-                                                     sv[4 * g + 2] << 16 | sv[4 * g + 3] << 24;
+            for (int g = 0; g < kQ; ++g) reinterpret_cast<uint32_t*>(cs)[g] = split_word(sv, g, true);
         } else if (cs) {
 #pragma unroll
-            for (int j = 0; j < kDecVPT; ++j) cs[j] = (uint8_t)sv[j];
+            for (int j = 0; j < kDecVPT; ++j)
+                cs[j] = (uint8_t)(split_word(sv, j >> 2, true) >> (8 * (j & 3)));
         }
     }
     return local;
@@ -579,6 +589,57 @@ constexpr unsigned kSmallThreads = 1024;
 constexpr unsigned kSmallSpan = kSmallThreads * kDecVPT;   // vertices per CTA: 8,192
 constexpr unsigned kSmallStage = 10240;                    // E[s] is about 1
 
+// The rest of k_decide_small where a factor of -1 or less (which no inference gives) has a count up to
+// 2^32 - 1: what the two passes make of it, whose totals hold the counts, chunk by chunk and
+// saturating, and whose emission reads the split bytes. A thread per chunk: as little code as it
+// takes, since code that is not run costs too (0.1 us of every decision; scans over the CTA here took 0.3).
+__device__ __forceinline__ void emit_odd(const DecideArgs& a, const Segment& sg,
+                                         const unsigned (&sv)[kDecVPT], bool whole,
+                                         uint32_t (&stage)[kSmallStage], unsigned (&chunk)[32],
+                                         unsigned& flags) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    constexpr unsigned kPer = kSmallSpan / kDecChunk;   // chunks per CTA
+    static_assert(kSmallStage >= kSmallSpan + kSmallSpan / 4 && 8 * kPer <= 32, "scratch");
+    const unsigned tid = threadIdx.x;
+#pragma unroll
+    for (int j = 0; j < kDecVPT; ++j) stage[kDecVPT * tid + j] = sv[j];
+#pragma unroll
+    for (int g = 0; g < kDecVPT / 4; ++g)
+        stage[kSmallSpan + kDecVPT / 4 * tid + g] = split_word(sv, g, whole);
+    __syncthreads();
+    if (tid < kPer) {
+        unsigned t = 0;
+#pragma unroll 1
+        for (unsigned k = 0; k < kDecChunk; ++k) t += stage[kDecChunk * tid + k];
+#pragma unroll 1
+        for (unsigned r = 0; r < gridDim.x; ++r)
+            *cluster.map_shared_rank(&chunk[kPer * blockIdx.x + tid], r) = t;
+    }
+    cluster.sync();
+    if (tid >= kPer) return;
+    unsigned long long before = 0, all = 0;
+#pragma unroll 1
+    for (unsigned k = 0; k < kPer * gridDim.x; ++k) {
+        if (k < kPer * blockIdx.x + tid) before += chunk[k];
+        all += chunk[k];
+    }
+    if (tid == 0 && blockIdx.x == 0) a.next_size[0] = all > ~0u ? ~0u : (unsigned)all;
+    const unsigned prefix = before > ~0u ? ~0u : (unsigned)before;
+    const unsigned room = prefix < sg.queue_capacity ? sg.queue_capacity - prefix : 0u;
+    uint32_t* q = a.queue + sg.queue_offset + prefix;
+    const uint8_t* bytes = reinterpret_cast<const uint8_t*>(stage + kSmallSpan) + kDecChunk * tid;
+    const unsigned first = sg.offset + (kPer * blockIdx.x + tid) * kDecChunk;
+    unsigned pos = 0;
+#pragma unroll 1
+    for (unsigned v = 0; v < kDecChunk; ++v)
+#pragma unroll 1
+        for (unsigned k = bytes[v]; k > 0; --k, ++pos) {
+            if (pos < room) q[pos] = a.sidx ? a.sidx[first + v] : first + v;
+            else flags |= NRRS_DEV_OVERFLOW;
+        }
+}
+
 __global__ void __launch_bounds__(kSmallThreads) k_decide_small(const __grid_constant__ DecideArgs a) {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
@@ -605,27 +666,38 @@ __global__ void __launch_bounds__(kSmallThreads) k_decide_small(const __grid_con
         const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += y;
     }
-    if (lane == 31) s_warp[wid] = incl;
+    unsigned most_sv = 0;
+#pragma unroll
+    for (int j = 0; j < kDecVPT; ++j) most_sv |= sv[j];
+    // a factor of -1 or less marks its warp, its CTA and so the cluster (counts sum to less than ~0)
+    const bool odd_warp = __any_sync(0xffffffffu, most_sv > 255u);
+    if (lane == 31) s_warp[wid] = odd_warp ? ~0u : incl;
     __syncthreads();
     cluster.barrier_wait(std::move(started));
     if (wid == 0) {
         unsigned w = s_warp[lane];
+        const bool odd = __any_sync(0xffffffffu, w == ~0u);
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const unsigned y = __shfl_up_sync(0xffffffffu, w, o);
             if (lane >= o) w += y;
         }
         s_warp[lane] = w;
-        const unsigned total = __shfl_sync(0xffffffffu, w, 31);
+        const unsigned total = odd ? ~0u : __shfl_sync(0xffffffffu, w, 31);
         if ((unsigned)lane < gridDim.x) *cluster.map_shared_rank(&s_tot[rank], lane) = total;
     }
     cluster.sync();   // every CTA has every total, and has read the sum
-    unsigned prefix = 0;
-    for (unsigned r = 0; r < rank; ++r) prefix += s_tot[r];   // at most 65,536 x 255 entries
+    if (tid == 0 && rank == 0) a.scr->sum_acc[0] = 0ull;   // restore the scratch
+    const unsigned of_lane = (unsigned)lane < gridDim.x ? s_tot[lane] : 0u;
+    const unsigned prefix = __reduce_add_sync(0xffffffffu, (unsigned)lane < rank ? of_lane : 0u);
+    if (__any_sync(0xffffffffu, of_lane == ~0u)) {
+        emit_odd(a, sg, sv, whole_run(a, v0, end), s_stage, s_warp, flags);
+        if (flags) atomicOr(&a.scr->status, flags);
+        return;
+    }
     const unsigned thread_excl = (wid ? s_warp[wid - 1] : 0) + incl - local;
     const unsigned total = s_warp[kSmallThreads / 32 - 1];
     if (tid == 0 && rank == gridDim.x - 1) a.next_size[0] = prefix + total;
-    if (tid == 0 && rank == 0) a.scr->sum_acc[0] = 0ull;   // restore the scratch
 
     uint32_t* q = a.queue + sg.queue_offset + prefix;
     const unsigned room = prefix < sg.queue_capacity ? sg.queue_capacity - prefix : 0u;

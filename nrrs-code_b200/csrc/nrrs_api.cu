@@ -1442,7 +1442,8 @@ int nrrs_autotune(nrrs_ctx* ctx, uint32_t n, const char* cache_path, char* repor
     const bool fp32 = c.precision == NRRS_PREC_FP32;
     // the FP32 path is timed as the steps run it, with features of the tuner's own
     FeatScratch feat{nullptr, segs.total_tiles < kF32PassTiles ? segs.total_tiles : kF32PassTiles};
-    if (fp32 && cudaMalloc(&feat.p, sizeof(float) * (size_t)kF32TileFloats * feat.tiles) != cudaSuccess) {
+    if (fp32 && ctx->feat &&
+        cudaMalloc(&feat.p, sizeof(float) * (size_t)kF32TileFloats * feat.tiles) != cudaSuccess) {
         feat.p = nullptr;
         cudaGetLastError();
     }
