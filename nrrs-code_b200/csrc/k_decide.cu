@@ -80,10 +80,21 @@ __device__ __forceinline__ float decide_scale(const DecideArgs& a, const Segment
     return a.scale_up ? nf : (nf < 1.0f ? nf : 1.0f);
 }
 
+__device__ __forceinline__ unsigned block_sum_u(unsigned v, unsigned* s_red) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    unsigned t = 0;
+#pragma unroll
+    for (int k = 0; k < kDecThreads / 32; ++k) t += s_red[k];
+    return t;
+}
+
 __global__ void __launch_bounds__(kDecThreads) k_decide(const __grid_constant__ DecideArgs a) {
     __shared__ unsigned s_chunk, s_epoch, s_prefix;
     __shared__ uint32_t s_stage[kDecStage];
-    __shared__ unsigned s_warp[kDecThreads / 32];
+    __shared__ unsigned s_warp[kDecThreads / 32], s_odd[kDecThreads / 32];
     const int tid = threadIdx.x;
     if (tid == 0) {
         s_chunk = atomicAdd(&a.scr->ticket, 1u);
@@ -175,16 +186,28 @@ __global__ void __launch_bounds__(kDecThreads) k_decide(const __grid_constant__ 
             }
         }
 
-        // block exclusive scan of the per-thread counts
+        // A factor of -1 or less (which no inference gives) has a count up to 2^32 - 1: the chunk's
+        // total holds it, but the copies are the split byte's, as in the two-pass emission
+        unsigned most_sv = 0;
+#pragma unroll
+        for (int j = 0; j < kDecVPT; ++j) most_sv |= sv[j];
+        unsigned copies = 0;
+#pragma unroll
+        for (int j = 0; j < kDecVPT; ++j) {
+            sv[j] = vec ? sp[j >> 2] >> (8 * (j & 3)) & 255u : sv[j] & 255u;
+            copies += sv[j];
+        }
+
+        // block exclusive scan of the per-thread copies
         const int lane = tid & 31, wid = tid >> 5;
-        unsigned incl = local;
+        unsigned incl = copies;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
             if (lane >= o) incl += y;
         }
         if (lane == 31) s_warp[wid] = incl;
-        __syncthreads();
+        const bool odd = __syncthreads_or(most_sv > 255u);
         if (wid == 0) {
             unsigned w = lane < kDecThreads / 32 ? s_warp[lane] : 0;
 #pragma unroll
@@ -196,8 +219,10 @@ __global__ void __launch_bounds__(kDecThreads) k_decide(const __grid_constant__ 
         }
         __syncthreads();
         const unsigned warp_excl = wid ? s_warp[wid - 1] : 0;
-        const unsigned thread_excl = warp_excl + incl - local;
-        const unsigned chunk_total = s_warp[kDecThreads / 32 - 1];
+        const unsigned thread_excl = warp_excl + incl - copies;
+        const unsigned chunk_copies = s_warp[kDecThreads / 32 - 1];
+        // (lane 0 of warp 0 has the total)
+        const unsigned chunk_total = odd ? block_sum_u(local, s_odd) : chunk_copies;
 
         // decoupled look-back by warp 0: each read covers the 32 chunks before a window top;
         // the closest inclusive prefix ends it, otherwise the window moves down by 32
@@ -263,13 +288,13 @@ __global__ void __launch_bounds__(kDecThreads) k_decide(const __grid_constant__ 
         // capacity, including a saturated prefix)
         uint32_t* q = a.queue + sg.queue_offset + s_prefix;
         const unsigned room = s_prefix < sg.queue_capacity ? sg.queue_capacity - s_prefix : 0u;
-        if (chunk_total <= kDecStage) {
+        if (chunk_copies <= kDecStage) {
             unsigned pos = thread_excl;
 #pragma unroll
             for (int j = 0; j < kDecVPT; ++j)
                 for (unsigned k = 0; k < sv[j]; ++k, ++pos) s_stage[pos] = st[j];
             __syncthreads();
-            for (unsigned e = tid; e < chunk_total; e += kDecThreads) {
+            for (unsigned e = tid; e < chunk_copies; e += kDecThreads) {
                 if (e < room) q[e] = s_stage[e];
                 else flags |= NRRS_DEV_OVERFLOW;
             }
@@ -312,17 +337,6 @@ __global__ void __launch_bounds__(kDecThreads) k_decide(const __grid_constant__ 
 // counts back (1 byte per vertex) and writes its queue entries at its prefix. Same decisions and
 // the same queue as the single-pass kernel, bit for bit; each CTA runs without waiting on any
 // other, which the single-pass kernel's per-chunk look-back and block barriers did.
-
-__device__ __forceinline__ unsigned block_sum_u(unsigned v, unsigned* s_red) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    unsigned t = 0;
-#pragma unroll
-    for (int k = 0; k < kDecThreads / 32; ++k) t += s_red[k];
-    return t;
-}
 
 // the split counts of chunk c, whose first vertex is `first`: the caller's array (indexed by
 // vertex), or the context's scratch, one kDecChunk-byte block per chunk (segment offsets are the

@@ -74,3 +74,24 @@ def test_odd_factors(net, n, few):
     got = host(queue, np.uint32)[:cap]
     assert np.array_equal(got[wrote == 1], want[wrote == 1])
     assert not got[wrote == 0].any()
+
+
+# the allocation-free entry point, on finite factors (its own sum scales: positive, below the budget)
+@pytest.mark.parametrize("n", [33, 2048, 5000, 30_001, 70_000])
+def test_odd_factors_noalloc(n):
+    torch = torch_cuda()
+    rng = np.random.default_rng(n)
+    rrs = rng.uniform(0.5, 8.0, n).astype(np.float32)
+    rrs[rng.choice(n, 5, replace=False)] = [-1.0, -1.5, -3.0, -7.25, -0.5]
+    rnd = rng.uniform(0.01, 0.99, n).astype(np.float32)
+    cap = 9 * n
+    norm, split, queue, size = empty(n), empty(n, "uint8"), empty(cap, "int32"), empty(1, "int32")
+    nb.decide_emit_noalloc(torch.from_numpy(rrs).cuda(), torch.from_numpy(rnd).cuda(), n, 1 << 30, 0,
+                           nb.default_decide(), norm, split, queue, cap, size, stream=stream())
+    nb.noalloc_device_status(stream())
+    b, want, wrote, total = expected(rrs, rnd, cap)
+    assert int(host(size, np.uint32)[0]) == total
+    assert np.array_equal(host(split)[:n], b)
+    got = host(queue, np.uint32)[:cap]
+    assert np.array_equal(got[wrote == 1], want[wrote == 1])
+    assert not got[wrote == 0].any()
